@@ -1548,9 +1548,10 @@ static vv_status prepare_frame(vv_renderer* r, const vv_frame_params& p, uint64_
         L.colors = r->tables.as<LabelTables>()->colors;
         L.scratch = r->mask_b.as<uint32_t>();
         L.out = r->mask_a.as<uint32_t>();
-        CK(launch_masks(L, st));
+        int launches = 0;
+        CK(launch_masks(L, st, &launches));
         r->prep_work = true;
-        r->launches += 4;
+        r->launches += launches;
         r->mask_key = key;
         r->have_mask_key = true;
     }

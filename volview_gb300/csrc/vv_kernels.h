@@ -74,7 +74,7 @@ enum {
 
 cudaError_t launch_density(const int16_t* hu, void* out, const Vol& v, cudaStream_t s);
 cudaError_t launch_normals(const void* d, uint32_t* out, const Vol& v, const m3& w2i, cudaStream_t s);
-cudaError_t launch_masks(const MaskLaunch& L, cudaStream_t s);
+cudaError_t launch_masks(const MaskLaunch& L, cudaStream_t s, int* launches);
 cudaError_t launch_majorant(const void* d, const uint32_t* mask, const Vol& v, int mode, float label_ext,
                             const float* bucket, float* out, cudaStream_t s);
 cudaError_t launch_unbrick(const void* src, void* dst, const Vol& v, int elem, cudaStream_t s);

@@ -533,6 +533,64 @@ __device__ Sample apply_labels(const PtArgs& A, Sample s, f3 idx) {
     return s;
 }
 
+// The label drawn at `idx` in the modes that draw labels alone (Isolate and
+// Hybrid; common.glsl:326-351): false where none is, so that the sample's
+// extinction is 0.
+__device__ __forceinline__ bool drawn_label(const PtArgs& A, f3 idx, uint32_t mode, uint32_t& label, bool& ghost) {
+    float2 m = mask_tri(A, idx);
+    ghost = m.x < (mode == 3u ? 0.25f : 0.5f);
+    if (ghost && !(m.y >= 0.5f)) return false;
+    return drawn_label_near(A, idx, mode, ghost, label);
+}
+// Whether with_label reads the CT density of a sample of `label`: only
+// Hybrid's opacity ramps do.
+__device__ __forceinline__ bool label_ramps(const PtArgs& A, uint32_t label, uint32_t mode, bool ghost) {
+    return mode == 3u && !ghost && __ldg(&A.tab->density[label].w) > 0.0f;
+}
+// The sample of `label` drawn at `idx` in those modes: with_label replaces
+// every field that the transfer function would give, so the transfer function
+// is not looked up, and the density is fetched only for a ramp.
+__device__ __forceinline__ Sample labelled_sample(const PtArgs& A, uint32_t label, uint32_t mode, bool ghost, float d) {
+    Sample s;
+    s.albedo = mk(0.0f);
+    s.extinction = 0.0f;
+    s.roughness = 0.0f;
+    s.metalness = 0.0f;
+    s.label = 0u;
+    s.ghost = false;
+    s.density = d;
+    s.subsurface = 0.0f;
+    s.coat = 0.0f;
+    return with_label(A, s, label, mode, ghost);
+}
+// apply_labels(tf_point(density), idx), with the fetches in an order that lets
+// most samples stop early: in the modes that draw labels alone the masks
+// decide first, and a sample outside them needs no density (64 taps in the
+// first flights) and no transfer function. What such a sample carries beside
+// its extinction of 0 is never read.
+template <bool CUBIC_ALLOWED>
+__device__ __forceinline__ Sample sample_labels(const PtArgs& A, f3 idx, bool cubic) {
+    const uint32_t mode = (uint32_t)A.u.labels[0];
+    if (mode >= 2u) {
+        uint32_t label;
+        bool ghost;
+        if (!drawn_label(A, idx, mode, label, ghost)) {
+            Sample s;
+            s.albedo = mk(0.0f);
+            s.extinction = 0.0f;
+            s.roughness = s.metalness = s.density = s.subsurface = s.coat = 0.0f;
+            s.label = 0u;
+            s.ghost = false;
+            return s;
+        }
+        float d = 0.0f;
+        if (label_ramps(A, label, mode, ghost)) d = CUBIC_ALLOWED && cubic ? density_cubic(A, idx) : density_tri(A, idx);
+        return labelled_sample(A, label, mode, ghost, d);
+    }
+    float d = CUBIC_ALLOWED && cubic ? density_cubic(A, idx) : density_tri(A, idx);
+    return apply_labels(A, tf_point(A, d), idx);
+}
+
 // common.glsl:357-373
 __device__ __forceinline__ float clip_depth(const PtArgs& A, f3 idx, int& plane) {
     plane = -1;
@@ -554,7 +612,7 @@ __device__ __forceinline__ float clip_depth(const PtArgs& A, f3 idx, int& plane)
 // sample_point (common.glsl:385-391) at an `idx` the caller has found inside
 // the kept part (clip_depth(idx) <= 0); clipped points have extinction 0.
 __device__ __forceinline__ Sample sample_point_unclipped(const PtArgs& A, f3 idx) {
-    Sample s = apply_labels(A, tf_point(A, density_tri(A, idx)), idx);
+    Sample s = sample_labels<false>(A, idx, false);
     if (s.ghost) s.extinction = 0.0f;
     return s;
 }
@@ -1082,8 +1140,7 @@ __device__ __noinline__ float bsdf_pdf(f3 n, f3 v, f3 l, const Sample& s) {
 // `idx` inside the kept part (cut = clip_depth(idx) <= 0).
 __device__ __noinline__ float extinction_unclipped(const PtArgs& A, f3 idx, f3 dir, bool smooth, Sample& s, int& cap_plane,
                                       float& cut) {
-    float d = (smooth && A.u.env[1] > 0.5f) ? density_cubic(A, idx) : density_tri(A, idx);
-    s = apply_labels(A, tf_point(A, d), idx);
+    s = sample_labels<true>(A, idx, smooth && A.u.env[1] > 0.5f);
     if (s.extinction <= 0.0f) return 0.0f;
     if (s.ghost) {
         f3 n;
@@ -1217,7 +1274,18 @@ __device__ __forceinline__ bool tr_step(const PtArgs& A, f3 origin, Shadow& T, R
     f3 q = origin + T.d_idx * T.tt;
     int plane;
     if (clip_depth(A, q, plane) > 0.0f) return true;
-    Sample m = sample_point_unclipped(A, q);
+    // Where no solid label is drawn the extinction is 0 (ghosts cast no shadow)
+    // and the estimate is multiplied by exactly 1.
+    const uint32_t mode = (uint32_t)A.u.labels[0];
+    Sample m;
+    if (mode >= 2u) {
+        uint32_t label;
+        if (mask_tri_ch(A, q, 0) < (mode == 3u ? 0.25f : 0.5f)) return true;
+        if (!drawn_label_near(A, q, mode, false, label)) return true;
+        m = labelled_sample(A, label, mode, false, label_ramps(A, label, mode, false) ? density_tri(A, q) : 0.0f);
+    } else {
+        m = sample_point_unclipped(A, q);
+    }
     T.result *= gmax(1.0f - path_sigma(A, m, m.extinction) / majorant, 0.0f);
     return true;
 }

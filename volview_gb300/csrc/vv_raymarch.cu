@@ -30,12 +30,17 @@ __device__ __forceinline__ void set3(f3& v, int i, float s) {
 __device__ __forceinline__ f3 index_to_tex(const PtArgs& A, f3 idx) { return (idx + 0.5f) / U3(A.u.dims); }
 __device__ __forceinline__ f3 tex_to_index(const PtArgs& A, f3 tex) { return tex * U3(A.u.dims) - 0.5f; }
 
-// common.glsl:385-391: a shadow-ray sample (ghosts and clipped parts cast no shadow).
+// common.glsl:385-391: a shadow-ray sample (ghosts and clipped parts cast no
+// shadow; a clipped point's other fields are not read).
 __device__ Sample sample_point(const PtArgs& A, f3 idx) {
-    Sample s = apply_labels(A, tf_point(A, density_tri(A, idx)), idx);
     int plane;
-    if (s.ghost || clip_depth(A, idx, plane) > 0.0f) s.extinction = 0.0f;
-    return s;
+    if (clip_depth(A, idx, plane) > 0.0f) {
+        Sample s;
+        s.albedo = mk(0.0f);
+        s.extinction = 0.0f;
+        return s;
+    }
+    return sample_point_unclipped(A, idx);
 }
 
 // common.glsl:160-162

@@ -650,13 +650,18 @@ __device__ __forceinline__ f3 brick_inv_dir(f3 d_idx) {
               1.0f / (d_idx.z == 0.0f ? 1e-9f : d_idx.z));
 }
 // brick_exit (common.glsl:430-436), multiplying by the ray's reciprocal
-// direction instead of dividing at every step.
-__device__ __forceinline__ float brick_exit(f3 idx, f3 inv_d) {
-    f3 lo = mk(floorf((idx.x + 0.5f) * 0.125f) * 8.0f - 0.5f, floorf((idx.y + 0.5f) * 0.125f) * 8.0f - 0.5f,
-               floorf((idx.z + 0.5f) * 0.125f) * 8.0f - 0.5f);
-    f3 hi = lo + 8.0f;
-    f3 t_far = gmax((lo - idx) * inv_d, (hi - idx) * inv_d);
-    return gmax(gmin(t_far.x, gmin(t_far.y, t_far.z)), 0.0f);
+// direction instead of dividing at every step. Per axis the larger of the two
+// planes' distances is that of the plane the ray runs towards: `far` (7.5 or
+// -0.5 voxels from the brick's first one, far_planes) picks it, and the plane's
+// position is exact in FP32 either way.
+__device__ __forceinline__ f3 far_planes(f3 inv_d) {
+    return mk(inv_d.x > 0.0f ? 7.5f : -0.5f, inv_d.y > 0.0f ? 7.5f : -0.5f, inv_d.z > 0.0f ? 7.5f : -0.5f);
+}
+__device__ __forceinline__ float brick_exit(f3 idx, f3 inv_d, f3 far) {
+    float tx = (fmaf(floorf((idx.x + 0.5f) * 0.125f), 8.0f, far.x) - idx.x) * inv_d.x;
+    float ty = (fmaf(floorf((idx.y + 0.5f) * 0.125f), 8.0f, far.y) - idx.y) * inv_d.y;
+    float tz = (fmaf(floorf((idx.z + 0.5f) * 0.125f), 8.0f, far.z) - idx.z) * inv_d.z;
+    return fmaxf(fminf(tx, fminf(ty, tz)), 0.0f);
 }
 
 // ------------------------------------------------------------ shading.glsl
@@ -1151,7 +1156,8 @@ __device__ __noinline__ float extinction_unclipped(const PtArgs& A, f3 idx, f3 d
 }
 
 // pt.comp:300-334: delta tracking against the brick majorants, hero channel,
-// as a resumable loop: ff_begin sets up the ray, each ff_step is one iteration.
+// as a resumable loop: ff_begin sets up the ray, ff_advance and ff_sample are
+// the halves of one iteration.
 struct Flight {
     f3 d_idx, inv_d;
     float tt, t_end;
@@ -1159,7 +1165,7 @@ struct Flight {
     int brick;    // brick whose flight majorant `maj` holds (-1: none yet)
     float maj;
 };
-enum { FF_CONTINUE = 0, FF_HIT = 1, FF_ESCAPE = 2 };
+enum { FF_CONTINUE = 0, FF_HIT = 1, FF_ESCAPE = 2, FF_SAMPLE = 4 };
 
 __device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Flight& F) {
     F.d_idx = mul(w2i3(A), dir);
@@ -1171,48 +1177,48 @@ __device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Fli
     F.brick = -1;
 }
 
-__device__ __forceinline__ int ff_step(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
-                                       Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
-    // The iterations of pt.comp:307-333 that fetch no voxel run back to back:
-    // empty bricks, samples beyond the brick exit, and tentative collisions in
-    // the clipped part (extinction_at returns 0 there before any fetch). The
-    // step ends at the first tentative collision that needs the volume. The
-    // majorant of the brick the ray is in is fetched once per brick.
-    float majorant;
-    for (;;) {
-        if (!(F.iter < 4096 && F.tt < F.t_end)) return FF_ESCAPE;
-        f3 p = origin + F.d_idx * F.tt;
-        int b = brick_index(A, p);
-        if (b != F.brick) {
-            F.brick = b;
-            F.maj = flight_majorant_of(A, b);
-        }
-        F.iter++;
-        majorant = F.maj;
-        float exit = F.tt + brick_exit(p, F.inv_d) + 1e-3f;
-        if (majorant <= 0.0f) {
-            F.tt = exit;
-            continue;
-        }
-        float next = F.tt - logf(1.0f - rng.rand()) / majorant;
-        if (next >= exit) {
-            F.tt = exit;
-            continue;
-        }
-        F.tt = next;
-        idx = origin + F.d_idx * F.tt;
-        cut = clip_depth(A, idx, cap_plane);
-        if (cut <= 0.0f) break;
+// One iteration of pt.comp:307-333 up to the voxel fetch. FF_CONTINUE: an
+// empty brick, a sample beyond the brick exit, or a tentative collision in the
+// clipped part (extinction_at returns 0 there before any fetch); FF_SAMPLE: a
+// tentative collision at F.tt that needs the volume (ff_sample); FF_ESCAPE.
+// The majorant of the brick the ray is in is fetched once per brick.
+__device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F, Rng& rng) {
+    if (!(F.iter < 4096 && F.tt < F.t_end)) return FF_ESCAPE;
+    f3 p = origin + F.d_idx * F.tt;
+    int b = brick_index(A, p);
+    if (b != F.brick) {
+        F.brick = b;
+        F.maj = flight_majorant_of(A, b);
     }
+    F.iter++;
+    float exit = F.tt + brick_exit(p, F.inv_d, far_planes(F.inv_d)) + 1e-3f;
+    if (F.maj <= 0.0f) {
+        F.tt = exit;
+        return FF_CONTINUE;
+    }
+    float next = F.tt - logf(1.0f - rng.rand()) / F.maj;
+    if (next >= exit) {
+        F.tt = exit;
+        return FF_CONTINUE;
+    }
+    F.tt = next;
+    int plane;
+    return clip_depth(A, origin + F.d_idx * F.tt, plane) <= 0.0f ? FF_SAMPLE : FF_CONTINUE;
+}
+// The rest of that iteration: the collision at F.tt, accepted (FF_HIT) or null.
+__device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
+                                         const Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
+    idx = origin + F.d_idx * F.tt;
+    cut = clip_depth(A, idx, cap_plane);
     float ext = extinction_unclipped(A, idx, dir, smooth, s, cap_plane, cut);
     if (ext <= 0.0f) return FF_CONTINUE;
     f3 sigma = path_sigma(A, s, ext);
     float sh = comp(sigma, hero);
-    if (rng.rand() * majorant < sh) {
+    if (rng.rand() * F.maj < sh) {
         spectral *= sigma / sh;
         return FF_HIT;
     }
-    spectral *= gmax(majorant - sigma, 0.0f) / (majorant - sh);
+    spectral *= gmax(F.maj - sigma, 0.0f) / (F.maj - sh);
     return FF_CONTINUE;
 }
 
@@ -1221,19 +1227,23 @@ __device__ bool free_flight(const PtArgs& A, f3 origin, f3 dir, bool smooth, int
     Flight F;
     ff_begin(A, origin, dir, F);
     for (;;) {
-        int r = ff_step(A, origin, dir, smooth, hero, spectral, F, idx, s, cap_plane, cut, rng);
+        int r = ff_advance(A, origin, F, rng);
+        if (r == FF_SAMPLE) r = ff_sample(A, origin, dir, smooth, hero, spectral, F, idx, s, cap_plane, cut, rng);
         if (r == FF_HIT) return true;
         if (r == FF_ESCAPE) return false;
     }
 }
 
-// pt.comp:339-371 as a resumable loop: tr_begin sets up the shadow ray, each
-// tr_step is one iteration; the estimate is in Shadow::result.
+// pt.comp:339-371 as a resumable loop: tr_begin sets up the shadow ray,
+// tr_advance and tr_sample are the halves of one iteration; the estimate is in
+// Shadow::result.
 struct Shadow {
     f3 d_idx, inv_d, result;
     float tt, t_end;
     int iter;
+    float maj;
 };
+enum { TR_CONTINUE = 0, TR_DONE = 1, TR_SAMPLE = 2 };
 __device__ __forceinline__ void tr_begin(const PtArgs& A, f3 origin, f3 dir, Shadow& T) {
     T.d_idx = mul(w2i3(A), dir);
     float2 tr = intersect_volume(A, origin, T.d_idx);
@@ -1243,59 +1253,61 @@ __device__ __forceinline__ void tr_begin(const PtArgs& A, f3 origin, f3 dir, Sha
     T.iter = 0;
     T.result = mk(1.0f);
 }
-// Returns false when the estimate is final.
-__device__ __forceinline__ bool tr_step(const PtArgs& A, f3 origin, Shadow& T, Rng& rng) {
-    // One iteration of pt.comp:345-370 per call. Samples in the clipped part
-    // need no fetch: sample_point's extinction is 0 there, path_sigma is 0 and
-    // the estimate is multiplied by exactly 1.
-    if (!(T.iter < 4096 && T.tt < T.t_end)) return false;
+// One iteration of pt.comp:345-370 up to the voxel fetch. TR_DONE: the
+// estimate is final; TR_SAMPLE: a sample at T.tt (tr_sample). Samples in the
+// clipped part need no fetch: sample_point's extinction is 0 there, path_sigma
+// is 0 and the estimate is multiplied by exactly 1.
+__device__ __forceinline__ int tr_advance(const PtArgs& A, f3 origin, Shadow& T, Rng& rng) {
+    if (!(T.iter < 4096 && T.tt < T.t_end)) return TR_DONE;
     T.iter++;
     float peak = maxc(T.result);
     if (peak < 0.1f) {
         if (rng.rand() * 0.1f >= peak) {
             T.result = mk(0.0f);
-            return false;
+            return TR_DONE;
         }
         T.result *= 0.1f / peak;
     }
     f3 p = origin + T.d_idx * T.tt;
-    float majorant = flight_majorant_of(A, brick_index(A, p));
-    float exit = T.tt + brick_exit(p, T.inv_d) + 1e-3f;
-    if (majorant <= 0.0f) {
+    T.maj = flight_majorant_of(A, brick_index(A, p));
+    float exit = T.tt + brick_exit(p, T.inv_d, far_planes(T.inv_d)) + 1e-3f;
+    if (T.maj <= 0.0f) {
         T.tt = exit;
-        return true;
+        return TR_CONTINUE;
     }
-    float next = T.tt - logf(1.0f - rng.rand()) / majorant;
+    float next = T.tt - logf(1.0f - rng.rand()) / T.maj;
     if (next >= exit) {
         T.tt = exit;
-        return true;
+        return TR_CONTINUE;
     }
     T.tt = next;
-    f3 q = origin + T.d_idx * T.tt;
     int plane;
-    if (clip_depth(A, q, plane) > 0.0f) return true;
-    // Where no solid label is drawn the extinction is 0 (ghosts cast no shadow)
-    // and the estimate is multiplied by exactly 1.
+    return clip_depth(A, origin + T.d_idx * T.tt, plane) > 0.0f ? TR_CONTINUE : TR_SAMPLE;
+}
+// The rest of that iteration: the sample at T.tt. Where no solid label is
+// drawn the extinction is 0 (ghosts cast no shadow) and the estimate is
+// multiplied by exactly 1.
+__device__ __forceinline__ void tr_sample(const PtArgs& A, f3 origin, Shadow& T) {
+    f3 q = origin + T.d_idx * T.tt;
     const uint32_t mode = (uint32_t)A.u.labels[0];
     Sample m;
     if (mode >= 2u) {
         uint32_t label;
-        if (mask_tri_ch(A, q, 0) < (mode == 3u ? 0.25f : 0.5f)) return true;
-        if (!drawn_label_near(A, q, mode, false, label)) return true;
+        if (mask_tri_ch(A, q, 0) < (mode == 3u ? 0.25f : 0.5f)) return;
+        if (!drawn_label_near(A, q, mode, false, label)) return;
         m = labelled_sample(A, label, mode, false, label_ramps(A, label, mode, false) ? density_tri(A, q) : 0.0f);
     } else {
         m = sample_point_unclipped(A, q);
     }
-    T.result *= gmax(1.0f - path_sigma(A, m, m.extinction) / majorant, 0.0f);
-    return true;
+    T.result *= gmax(1.0f - path_sigma(A, m, m.extinction) / T.maj, 0.0f);
 }
 
 // pt.comp:339-371: ratio tracking with Russian roulette.
 __device__ __noinline__ f3 transmittance(const PtArgs& A, f3 origin, f3 dir, Rng& rng) {
     Shadow T;
     tr_begin(A, origin, dir, T);
-    while (tr_step(A, origin, T, rng)) {
-    }
+    for (int r; (r = tr_advance(A, origin, T, rng)) != TR_DONE;)
+        if (r == TR_SAMPLE) tr_sample(A, origin, T);
     return T.result;
 }
 

@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_cons
             f3 idx = o_idx + d_idx * tt;
             float maj = A.u.path[3] == 0u ? 1e30f : __ldg(A.majorant + brick_index(A, idx));
             if (maj <= 0.0f) {
-                tt += brick_exit(idx, inv_d);
+                tt += brick_exit(idx, inv_d, far_planes(inv_d));
                 prev_density = -1.0f;
                 continue;
             }

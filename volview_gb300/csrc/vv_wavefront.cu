@@ -426,28 +426,41 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
     }
 }
 
-// Extend, persistent over its queue: every lane advances its path by one
-// free-flight step per iteration; a lane whose flight ended (a vertex, an
-// escape, or the bounce limits) hands the path on and takes the next queued
-// path, so lanes with long empty-space flights do not hold up the others.
-// ff_step is the loop body of free_flight (pt.comp:307-332). Only what the
-// flight needs stays in registers. Vertices go to shade; escapes and paths at
-// the bounce limits go to this wave's scatter kernel, which finishes them, so
-// this kernel carries none of the escape, accumulation or path-start code.
+// Extend, persistent over its queue: a warp takes 32 queued paths (neighbours in
+// the image, or in a bin), flies them all to their ends, writes them out and
+// takes the next 32. A flight is two pieces of code: an advance through a brick
+// (ff_advance, about 60 instructions) and a sample of the volume (ff_sample,
+// several hundred and more for ghosts). The warp runs them as phases: lanes
+// that reach a tentative collision wait until VV_EXTEND_GATHER of them have, or
+// no lane advances any more, and then sample together. Bound by instruction
+// issue and fetch on divergent warps. Measured at 16 frames of 1024^2 per pass
+// (head/neck, passes overlapping), against a loop that advanced every lane to
+// its next collision, sampled at once and refilled ended lanes (394 M path
+// samples/s): phases with single-lane refill 327, refill at 8 ended lanes 476,
+// at 16 507-511, with all 32 ended 531-534. A refilled lane starts in the empty
+// bricks around the volume, or in another bin, and the other lanes wait through
+// its steps. VV_EXTEND_GATHER 12, 16, 20, 24, 28: 528, 532, 531, 530, 526.
+// Vertices go to shade; escapes and paths at the bounce limits go to this wave's
+// scatter kernel, which finishes them, so this kernel carries none of the
+// escape, accumulation or path-start code.
 #ifndef VV_EXTEND_MIN_BLOCKS
 #define VV_EXTEND_MIN_BLOCKS 8
 #endif
+#ifndef VV_EXTEND_GATHER
+#define VV_EXTEND_GATHER 20
+#endif
 enum { EXT_END = 3 };
+enum { LANE_OUT, LANE_ADVANCE, LANE_SAMPLE };
 // FIRST: the first-flight queue (bounce 0: cubic B-spline density along the
 // flight), otherwise later flights (trilinear); each kernel carries only its
-// sampler. Every wave launches both; with all of a pass's frames in flight
-// first flights occur in the first wave only (and with several samples per
-// pixel), so the other launch finds its queue empty.
+// sampler. With all of a pass's items in flight and one sample per pixel, first
+// flights occur in the first wave only, and the other waves launch the second
+// kernel alone. `leads`: the wave's first launch.
 template <bool FIRST, class X>
 __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
-    k_wf_extend(const __grid_constant__ X B, const WfArgs W, int cur, uint32_t tail) {
+    k_wf_extend(const __grid_constant__ X B, const WfArgs W, int cur, uint32_t tail, int leads) {
     if (W.counts[WF_STOP] != 0u) return;
-    if (FIRST) {
+    if (leads) {
         // The wave's first launch decides whether the waves go on: with at most
         // `tail` live paths left, the finishing launch takes queue `cur` over.
         // Every block reads the same counts (nothing changes them before this
@@ -468,65 +481,75 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
     uint32_t word = 0;  // P2.w: volumes, sample, hero
     Flight F;
     Vertex V;
-    bool active = false, drained = false;
     for (;;) {
-        int done = 0;
-        bool need = !active && !drained;
-        if (__any_sync(0xffffffffu, need)) {
-            uint32_t k = take_item(taken, n, need);
-            if (need && k != ~0u) {
-                slot = queue[k];
-                r = request_of(B, slot);
-                const PtArgs& A = args_of(B, r);
-                const Consts& C = consts_of(B, W, r, C0);
-                const float4* q = rec(W.path, slot, PATH_N);
-                float4 a = q[0], b = q[1], c = q[2];
-                origin = xyz(a);
-                rng.s = ubits(a.w);
-                dir = xyz(b);
-                spectral = xyz(c);
-                word = ubits(c.w);
-                uint32_t surfaces = ubits(b.w) >> 16, volumes = word & 1023u;
-                if (!(surfaces <= C.max_bounces && volumes <= C.volume_limit)) {
-                    done = EXT_END;
-                } else {
-                    count(A, COUNT_VERTEX);
-                    ff_begin(A, origin, dir, F);
-                    active = true;
-                }
-            }
-            drained = __any_sync(0xffffffffu, need && k == ~0u);
-        }
-        if (active) {
-            int res = ff_step(args_of(B, r), origin, dir, FIRST, (int)(word >> 30), spectral, F, V.idx, V.s,
-                              V.cap_plane, V.cut, rng);
-            if (res != FF_CONTINUE) {
-                active = false;
-                done = res;
+        const uint32_t k = take_item(taken, n, true);
+        int state = LANE_OUT, result = EXT_END;
+        if (!__any_sync(0xffffffffu, k != ~0u)) break;
+        if (k != ~0u) {
+            slot = queue[k];
+            r = request_of(B, slot);
+            const PtArgs& A = args_of(B, r);
+            const Consts& C = consts_of(B, W, r, C0);
+            const float4* q = rec(W.path, slot, PATH_N);
+            float4 a = q[0], b = q[1], c = q[2];
+            origin = xyz(a);
+            rng.s = ubits(a.w);
+            dir = xyz(b);
+            spectral = xyz(c);
+            word = ubits(c.w);
+            uint32_t surfaces = ubits(b.w) >> 16, volumes = word & 1023u;
+            if (surfaces <= C.max_bounces && volumes <= C.volume_limit) {
+                count(A, COUNT_VERTEX);
+                ff_begin(A, origin, dir, F);
+                state = LANE_ADVANCE;
             }
         }
-        if (__any_sync(0xffffffffu, done != 0)) {
-            if (done != 0) {
-                if (done != EXT_END) {  // free flight changed the spectral ratios
-                    float4* q = rec(W.path, slot, PATH_N);
-                    float4 d = q[3];
-                    q[2] = f4(spectral, fbits(word));
-                    q[3] = d;
-                }
-                float4* v = rec(W.vtx, slot, VTX_N);
-                if (done == FF_HIT) {
-                    store_vertex(W, slot, V, rng.s);
-                } else {
-                    // Escapes and paths at the bounce limits: the random state
-                    // and whether the scatter kernel runs the escape (pt.comp:431-447).
-                    v[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    v[3] = make_float4(0.0f, 0.0f, fbits(rng.s), fbits(done == FF_ESCAPE ? 1u : 0u));
+        for (;;) {
+            // Advance until enough lanes wait for a sample, or all the rest has ended.
+            unsigned sampling;
+            for (;;) {
+                const unsigned advancing = __ballot_sync(0xffffffffu, state == LANE_ADVANCE);
+                sampling = __ballot_sync(0xffffffffu, state == LANE_SAMPLE);
+                if (!advancing || __popc(sampling) >= VV_EXTEND_GATHER) break;
+                if (state == LANE_ADVANCE) {
+                    const int res = ff_advance(args_of(B, r), origin, F, rng);
+                    if (res == FF_SAMPLE) state = LANE_SAMPLE;
+                    if (res == FF_ESCAPE) {
+                        state = LANE_OUT;
+                        result = FF_ESCAPE;
+                    }
                 }
             }
-            push(W.shade, &W.counts[WF_SHADE], slot, done == FF_HIT);
-            push(W.esc[cur], &W.counts[WF_ESC0 + cur], slot, done != 0 && done != FF_HIT);
+            if (!sampling) break;
+            if (state == LANE_SAMPLE) {
+                const int res = ff_sample(args_of(B, r), origin, dir, FIRST, (int)(word >> 30), spectral, F, V.idx,
+                                          V.s, V.cap_plane, V.cut, rng);
+                state = LANE_ADVANCE;
+                if (res == FF_HIT) {
+                    state = LANE_OUT;
+                    result = FF_HIT;
+                }
+            }
         }
-        if (drained && !__any_sync(0xffffffffu, active)) break;
+        if (k != ~0u) {
+            if (result != EXT_END) {  // free flight changed the spectral ratios
+                float4* q = rec(W.path, slot, PATH_N);
+                float4 d = q[3];
+                q[2] = f4(spectral, fbits(word));
+                q[3] = d;
+            }
+            float4* v = rec(W.vtx, slot, VTX_N);
+            if (result == FF_HIT) {
+                store_vertex(W, slot, V, rng.s);
+            } else {
+                // Escapes and paths at the bounce limits: the random state
+                // and whether the scatter kernel runs the escape (pt.comp:431-447).
+                v[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                v[3] = make_float4(0.0f, 0.0f, fbits(rng.s), fbits(result == FF_ESCAPE ? 1u : 0u));
+            }
+        }
+        push(W.shade, &W.counts[WF_SHADE], slot, k != ~0u && result == FF_HIT);
+        push(W.esc[cur], &W.counts[WF_ESC0 + cur], slot, k != ~0u && result != FF_HIT);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) W.counts[WF_SCATTER] = 0;
 }
@@ -569,13 +592,27 @@ __global__ void __launch_bounds__(128, VV_SHADE_MIN_BLOCKS) k_wf_shade(const __g
     }
 }
 
-// Shadow rays, persistent over their queue like extend: one ratio-tracking
-// step (tr_step, the loop body of transmittance, pt.comp:344-369) per
-// iteration, lanes refilled as their rays finish. With a light map, a lane
-// whose key-light ray finished draws the light map's sample (pt.comp:466-476,
-// in the reference's order of random numbers) and queues the slot for
-// k_wf_shadow_map, which traces the sample's ray: a lane here traces one kind
-// of ray, and the random state travels in the shadow record between them.
+// The warp's shadow rays (the lanes with `active` set) to their ends, in step:
+// an advance of all of them, then the samples of those that need one.
+__device__ __forceinline__ void trace_shadows(const PtArgs& A, bool active, f3 origin, Shadow& T, Rng& rng) {
+    while (__any_sync(0xffffffffu, active)) {
+        int res = TR_CONTINUE;
+        if (active) res = tr_advance(A, origin, T, rng);
+        active = active && res != TR_DONE;
+        __syncwarp();
+        if (res == TR_SAMPLE) tr_sample(A, origin, T);
+    }
+}
+
+// Shadow rays, persistent over their queue like extend, 32 at a time. A sample
+// here is shorter than an advance, so it follows its advance at once (gathering
+// 2, 4 or 6 lanes first: 528, 511, 500 M path samples/s against 535); refilling
+// lanes one by one or at 4, 8, 16, 24 ended ones ran at 510, 516, 522, 528 and
+// 528. With a light map, a lane whose key-light ray finished draws the light
+// map's sample (pt.comp:466-476, in the reference's order of random numbers)
+// and queues the slot for k_wf_shadow_map, which traces the sample's ray: a
+// lane here traces one kind of ray, and the random state travels in the shadow
+// record between them.
 #ifndef VV_SHADOW_MIN_BLOCKS
 #define VV_SHADOW_MIN_BLOCKS 8
 #endif
@@ -590,32 +627,27 @@ __global__ void __launch_bounds__(128, VV_SHADOW_MIN_BLOCKS) k_wf_shadow(const _
     f3 origin;
     Rng rng;
     Shadow T;
-    bool active = false, drained = false;
     for (;;) {
-        bool need = !active && !drained;
-        if (__any_sync(0xffffffffu, need)) {
-            uint32_t k = take_item(&W.counts[WF_TAKE_SHADOW], n, need);
-            if (need && k != ~0u) {
-                slot = W.shadow[k];
-                r = request_of(B, slot);
-                const float4* q = rec(W.shd, slot, SHD_N);
-                float4 a = q[0], b = q[1];
-                origin = xyz(a);
-                rng.s = ubits(a.w);
-                tr_begin(args_of(B, r), origin, xyz(b), T);
-                active = true;
-            }
-            drained = __any_sync(0xffffffffu, need && k == ~0u);
+        const uint32_t k = take_item(&W.counts[WF_TAKE_SHADOW], n, true);
+        if (!__any_sync(0xffffffffu, k != ~0u)) break;
+        bool done = k != ~0u, to_map = false;
+        if (done) {
+            slot = W.shadow[k];
+            r = request_of(B, slot);
+            const float4* q = rec(W.shd, slot, SHD_N);
+            float4 a = q[0], b = q[1];
+            origin = xyz(a);
+            rng.s = ubits(a.w);
+            tr_begin(args_of(B, r), origin, xyz(b), T);
         }
-        bool done = false, to_map = false;
-        if (active && !tr_step(args_of(B, r), origin, T, rng)) {
+        trace_shadows(args_of(B, r), done, origin, T, rng);
+        if (done) {
             const PtArgs& A = args_of(B, r);
             const bool map = MAP && (!IsBatch<X>::value || A.u.lighting[3] == 2u);
             float4* h = rec(W.sh, slot, SH_N);
             if (!map) {
                 h[0] = f4(T.result, fbits(rng.s));
                 h[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                done = true;
             } else {
                 Vertex V;
                 sample_map_light(A, rng, V);
@@ -625,11 +657,10 @@ __global__ void __launch_bounds__(128, VV_SHADOW_MIN_BLOCKS) k_wf_shadow(const _
                 to_map = V.map_pdf > 0.0f;
                 done = !to_map;
             }
-            active = false;
         }
+        __syncwarp();
         if (MAP) push(W.map, &W.counts[WF_MAP], slot, to_map);
-        if (__any_sync(0xffffffffu, done)) push(W.scatter, &W.counts[WF_SCATTER], slot, done);
-        if (drained && !__any_sync(0xffffffffu, active)) break;
+        push(W.scatter, &W.counts[WF_SCATTER], slot, done);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) W.counts[WF_SHADE] = 0;
 }
@@ -647,32 +678,25 @@ __global__ void __launch_bounds__(128, VV_SHADOW_MIN_BLOCKS) k_wf_shadow_map(con
     f3 origin;
     Rng rng;
     Shadow T;
-    bool active = false, drained = false;
     for (;;) {
-        bool need = !active && !drained;
-        if (__any_sync(0xffffffffu, need)) {
-            uint32_t k = take_item(&W.counts[WF_TAKE_MAP], n, need);
-            if (need && k != ~0u) {
-                slot = W.map[k];
-                r = request_of(B, slot);
-                origin = xyz(rec(W.shd, slot, SHD_N)[0]);
-                rng.s = ubits(rec(W.sh, slot, SH_N)[0].w);
-                tr_begin(args_of(B, r), origin, xyz(W.mapdir[slot]), T);
-                active = true;
-            }
-            drained = __any_sync(0xffffffffu, need && k == ~0u);
+        const uint32_t k = take_item(&W.counts[WF_TAKE_MAP], n, true);
+        if (!__any_sync(0xffffffffu, k != ~0u)) break;
+        if (k != ~0u) {
+            slot = W.map[k];
+            r = request_of(B, slot);
+            origin = xyz(rec(W.shd, slot, SHD_N)[0]);
+            rng.s = ubits(rec(W.sh, slot, SH_N)[0].w);
+            tr_begin(args_of(B, r), origin, xyz(W.mapdir[slot]), T);
         }
-        bool done = false;
-        if (active && !tr_step(args_of(B, r), origin, T, rng)) {
+        trace_shadows(args_of(B, r), k != ~0u, origin, T, rng);
+        if (k != ~0u) {
             float4* h = rec(W.sh, slot, SH_N);
             float4 h0 = h[0], h1 = h[1];
             h[0] = make_float4(h0.x, h0.y, h0.z, fbits(rng.s));
             h[1] = f4(xyz(h1) * T.result, h1.w);
-            done = true;
-            active = false;
         }
-        if (__any_sync(0xffffffffu, done)) push(W.scatter, &W.counts[WF_SCATTER], slot, done);
-        if (drained && !__any_sync(0xffffffffu, active)) break;
+        __syncwarp();
+        push(W.scatter, &W.counts[WF_SCATTER], slot, k != ~0u);
     }
 }
 
@@ -793,24 +817,21 @@ __global__ void __launch_bounds__(256) k_wf_bin_place(const WfArgs W, const uint
     }
 }
 
-// The paths still alive, run to completion one thread each (the reference's
-// loop), including their pixels' remaining samples and frames (a batched
-// pass's from each path's own request).
+// The paths still alive, run to completion (the reference's loop), including
+// their pixels' remaining samples and frames (a batched pass's from each path's
+// own request). Each runs alone in a warp, which takes the next one when it
+// ends: 32 divergent random walks to a warp take turns through each other's
+// code, and 2 or 4 to a warp finish no sooner.
 template <class X>
 __global__ void __launch_bounds__(128, 4) k_wf_finish(const __grid_constant__ X B, const WfArgs W, int cur) {
     uint32_t stop = W.counts[WF_STOP];
     if (stop != 0u) cur = (int)stop - 1;  // else the waves ran out first: `cur` is the next wave's queue
     uint32_t n_first = W.counts[WF_FIRST0 + cur], n = n_first + W.counts[cur];
     const Consts C0 = kernel_consts(B);
-    // With no more paths than warps (the usual tail: at most 1024 paths), each
-    // path runs alone in its warp, on every SM, instead of 32 to a warp on a
-    // few SMs, where the lanes would take turns through each other's divergent
-    // random walks. More paths (the waves ran out first) take a lane each.
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
-    const bool alone = n <= (threads >> 5);
-    if (alone && (threadIdx.x & 31u) != 0u) return;
-    const uint32_t first = alone ? tid >> 5 : tid, stride = alone ? threads >> 5 : threads;
-    for (uint32_t i = first; i < n; i += stride) {
+    if ((threadIdx.x & 31u) != 0u) return;
+    for (;;) {
+        const uint32_t i = atomicAdd(&W.counts[WF_TAKE_EXT], 1u);  // zero: the last wave's shade cleared it
+        if (i >= n) break;
         uint32_t slot = i < n_first ? W.first[cur][i] : W.ext[cur][i - n_first];
         const uint32_t r = request_of(B, slot);
         const PtArgs& A = args_of(B, r);
@@ -851,7 +872,7 @@ template <class K> static int blocks_per_sm(K kernel, int threads) {
 // of the four stages until few paths are left, then one finishing launch.
 template <class X>
 static cudaError_t run_waves(const X& a, const WfArgs& w, int sms, cudaStream_t s, int* launches, uint32_t slots,
-                             uint32_t rounds, bool map) {
+                             uint32_t rounds, bool refills, bool map) {
     static int g_ext = 0, g_shade = 0, g_shadow = 0, g_scatter = 0, g_finish = 0;
     if (!g_ext) {
         g_ext = sms * blocks_per_sm(k_wf_extend<false, X>, 128);
@@ -880,8 +901,12 @@ static cudaError_t run_waves(const X& a, const WfArgs& w, int sms, cudaStream_t 
     int waves = (int)std::min<uint32_t>(first + 10u * rounds, 4096u);
     int cur = 0;
     for (int wave = 0; wave < waves; wave++) {
-        k_wf_extend<true, X><<<g_ext, 128, 0, s>>>(a, w, cur, tail);
-        k_wf_extend<false, X><<<g_ext, 128, 0, s>>>(a, w, cur, tail);
+        // Launches that would find nothing to do are left out: first flights
+        // after the first wave of a pass without refills, later flights in the
+        // first wave, the ordering of queues that cannot reach bin_min.
+        const bool first_flights = wave == 0 || refills;
+        if (first_flights) k_wf_extend<true, X><<<g_ext, 128, 0, s>>>(a, w, cur, tail, 1);
+        if (wave > 0) k_wf_extend<false, X><<<g_ext, 128, 0, s>>>(a, w, cur, tail, !first_flights);
         k_wf_shade<X><<<g_shade, 128, 0, s>>>(a, w, cur);
         if (map) {
             k_wf_shadow<true, X><<<g_shadow, 128, 0, s>>>(a, w);
@@ -891,13 +916,14 @@ static cudaError_t run_waves(const X& a, const WfArgs& w, int sms, cudaStream_t 
             k_wf_shadow<false, X><<<g_shadow, 128, 0, s>>>(a, w);
         }
         k_wf_scatter<X><<<g_scatter, 128, 0, s>>>(a, w, cur);
-        *launches += 5;
-        // The next wave's later flights, ordered by bin.
-        k_wf_bin_count<<<sms * 4, 256, 0, s>>>(w, w.ext_key[cur ^ 1], cur ^ 1);
-        k_wf_bin_scan<<<1, 1024, 0, s>>>(w, cur ^ 1);
-        k_wf_bin_place<<<sms * 4, 256, 0, s>>>(w, w.ext[cur ^ 1], w.ext_key[cur ^ 1], cur ^ 1);
-        *launches += 3;
+        *launches += 3 + first_flights + (wave > 0);
         cur ^= 1;
+        if (slots < w.bin_min) continue;
+        // The next wave's later flights, ordered by bin.
+        k_wf_bin_count<<<sms * 4, 256, 0, s>>>(w, w.ext_key[cur], cur);
+        k_wf_bin_scan<<<1, 1024, 0, s>>>(w, cur);
+        k_wf_bin_place<<<sms * 4, 256, 0, s>>>(w, w.ext[cur], w.ext_key[cur], cur);
+        *launches += 3;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -913,7 +939,7 @@ cudaError_t launch_pt_wavefront(const PtArgs& a, const WfArgs& w, int sms, cudaS
     uint32_t items = a.frames * pixels;
     uint32_t slots = items < w.capacity ? items : w.capacity;  // paths in flight
     uint32_t rounds = (items + slots - 1) / slots;
-    return run_waves(a, w, sms, s, launches, slots, rounds, a.u.lighting[3] == 2u);
+    return run_waves(a, w, sms, s, launches, slots, rounds, rounds > 1u || a.u.path[2] > 1u, a.u.lighting[3] == 2u);
 }
 
 #if VV_DFMT == 0
@@ -923,7 +949,7 @@ cudaError_t launch_pt_wavefront(const PtArgs& a, const WfArgs& w, int sms, cudaS
 cudaError_t launch_pt_wavefront_batch(const PtBatch& b, const WfArgs& w, int sms, cudaStream_t s, int* launches) {
     if (b.n == 0 || b.n > (uint32_t)VV_BATCH_MAX || !w.items || !w.consts) return cudaErrorInvalidValue;
     uint32_t rounds = 1, begin = 0;
-    bool map = false;
+    bool map = false, refills = false;
     for (uint32_t r = 0; r < b.n; r++) {
         const PtArgs& a = b.a[r];
         if (a.u.path[2] >= (uint32_t)WF_MAX_SAMPLES) return cudaErrorInvalidValue;
@@ -931,10 +957,11 @@ cudaError_t launch_pt_wavefront_batch(const PtBatch& b, const WfArgs& w, int sms
         if (b.slot_end[r] <= begin || slots > items) return cudaErrorInvalidValue;
         rounds = std::max(rounds, (items + slots - 1) / slots);
         map = map || a.u.lighting[3] == 2u;
+        refills = refills || items > slots || a.u.path[2] > 1u;
         begin = b.slot_end[r];
     }
     if (begin > w.capacity) return cudaErrorInvalidValue;
-    return run_waves(b, w, sms, s, launches, begin, rounds, map);
+    return run_waves(b, w, sms, s, launches, begin, rounds, refills, map);
 }
 #endif
 

@@ -777,21 +777,47 @@ __device__ __forceinline__ f3 hash3(int cx, int cy, int cz) {
     const float s = 1.0f / 4294967296.0f;
     return mk((float)x * s, (float)y * s, (float)z * s);
 }
-__device__ __forceinline__ float gradient_at(int cx, int cy, int cz, f3 off) {
-    f3 h = hash3(cx, cy, cz);
-    return dot(h * 2.0f - 1.0f, off);
+// The gradient vectors at the eight corners of lattice cell (ix, iy, iz), and
+// the noise they give at a point of the cell, `f` its offset in it
+// (shading.glsl:192-202).
+struct Lattice {
+    f3 g[8];  // x fastest
+};
+__device__ __forceinline__ Lattice lattice_at(int ix, int iy, int iz) {
+    Lattice l;
+#pragma unroll
+    for (int k = 0; k < 8; k++) l.g[k] = hash3(ix + (k & 1), iy + ((k >> 1) & 1), iz + (k >> 2)) * 2.0f - 1.0f;
+    return l;
 }
-// shading.glsl:192-202
+// Sums of products rounded one way wherever they are inlined (a noise must not
+// depend on whether its cell's vectors were shared): fused as the compiler
+// contracts them in a lone gradient_noise, unfused in the parity build.
+__device__ __forceinline__ float two_products(float a, float b, float c, float d) {
+#if VV_EXACT
+    return a * b + c * d;
+#else
+    return fmaf(a, b, __fmul_rn(c, d));
+#endif
+}
+__device__ __forceinline__ float lattice_dot(f3 a, f3 b) {
+#if VV_EXACT
+    return dot(a, b);
+#else
+    return fmaf(a.z, b.z, two_products(a.x, b.x, a.y, b.y));
+#endif
+}
+__device__ __forceinline__ float lattice_mix(float x, float y, float a) { return two_products(x, 1.0f - a, y, a); }
+__device__ __forceinline__ float lattice_noise(const Lattice& l, f3 f) {
+    f3 w = f * f * f * (f * (f * 6.0f - 15.0f) + 10.0f);
+    float x00 = lattice_mix(lattice_dot(l.g[0], f), lattice_dot(l.g[1], f - mk(1, 0, 0)), w.x);
+    float x10 = lattice_mix(lattice_dot(l.g[2], f - mk(0, 1, 0)), lattice_dot(l.g[3], f - mk(1, 1, 0)), w.x);
+    float x01 = lattice_mix(lattice_dot(l.g[4], f - mk(0, 0, 1)), lattice_dot(l.g[5], f - mk(1, 0, 1)), w.x);
+    float x11 = lattice_mix(lattice_dot(l.g[6], f - mk(0, 1, 1)), lattice_dot(l.g[7], f - mk(1, 1, 1)), w.x);
+    return 1.7f * lattice_mix(lattice_mix(x00, x10, w.y), lattice_mix(x01, x11, w.y), w.z);
+}
 __device__ __noinline__ float gradient_noise(f3 p) {
     float flx = floorf(p.x), fly = floorf(p.y), flz = floorf(p.z);
-    int ix = (int)flx, iy = (int)fly, iz = (int)flz;
-    f3 f = mk(p.x - flx, p.y - fly, p.z - flz);
-    f3 w = f * f * f * (f * (f * 6.0f - 15.0f) + 10.0f);
-    float x00 = mixf(gradient_at(ix, iy, iz, f), gradient_at(ix + 1, iy, iz, f - mk(1, 0, 0)), w.x);
-    float x10 = mixf(gradient_at(ix, iy + 1, iz, f - mk(0, 1, 0)), gradient_at(ix + 1, iy + 1, iz, f - mk(1, 1, 0)), w.x);
-    float x01 = mixf(gradient_at(ix, iy, iz + 1, f - mk(0, 0, 1)), gradient_at(ix + 1, iy, iz + 1, f - mk(1, 0, 1)), w.x);
-    float x11 = mixf(gradient_at(ix, iy + 1, iz + 1, f - mk(0, 1, 1)), gradient_at(ix + 1, iy + 1, iz + 1, f - mk(1, 1, 1)), w.x);
-    return 1.7f * mixf(mixf(x00, x10, w.y), mixf(x01, x11, w.y), w.z);
+    return lattice_noise(lattice_at((int)flx, (int)fly, (int)flz), mk(p.x - flx, p.y - fly, p.z - flz));
 }
 __device__ float fbm(f3 p) {
     return (gradient_noise(p) + 0.5f * gradient_noise(p * 2.03f + 17.1f) + 0.25f * gradient_noise(p * 4.07f + 31.7f)) /
@@ -824,14 +850,11 @@ __device__ float lobule_border(f3 q, int lobule[3]) {
     cellular(q + 0.2f * warp, nearest, border, lobule);
     return border;
 }
-__device__ __noinline__ float surface_height(f3 p, float4 params) {
+__device__ __noinline__ float lobule_height(f3 p, float4 params) {
     f3 q = p / params.w;
-    if (params.x > 1.5f) {
-        int lobule[3];
-        float bulge = smoothstepf(0.0f, 0.35f, lobule_border(q, lobule));
-        return 0.7f * bulge + 0.3f * fbm(q * 3.0f);
-    }
-    return 0.6f * fbm(q) + 0.4f * gradient_noise(q * 4.0f);
+    int lobule[3];
+    float bulge = smoothstepf(0.0f, 0.35f, lobule_border(q, lobule));
+    return 0.7f * bulge + 0.3f * fbm(q * 3.0f);
 }
 // shading.glsl:263-265: inverse(mat3(world_to_index)) * (idx - translation).
 __device__ __noinline__ f3 index_to_world(const PtArgs& A, f3 idx) {
@@ -848,12 +871,19 @@ __device__ __noinline__ f3 index_to_world(const PtArgs& A, f3 idx) {
 __device__ __forceinline__ bool textured(const PtArgs& A, const Sample& s) {
     return s.label != 0u && !s.ghost && __ldg(&A.tab->surface[s.label].x) > 0.5f;
 }
+// What the relief at a point shares with its texture: the point in world space
+// and, but for lobules (params.x > 1.5), the two noises of its height.
+struct SurfaceNoise {
+    f3 p;
+    float patches, grain;
+};
 // shading.glsl:273-324
-__device__ __noinline__ void apply_surface_texture(const PtArgs& A, f3 idx, Sample& s) {
+__device__ __noinline__ void apply_surface_texture(const PtArgs& A, f3 idx, Sample& s, SurfaceNoise& noise) {
     if (!textured(A, s)) return;
     float4 params = ldf4(&A.tab->surface[s.label]);
     float amount = params.y;
     f3 p = index_to_world(A, idx);
+    noise.p = p;
     f3 q = p / params.w;
     f3 tint;
     float wet, rough;
@@ -880,6 +910,8 @@ __device__ __noinline__ void apply_surface_texture(const PtArgs& A, f3 idx, Samp
     } else {
         float patches = fbm(q);
         float grain = gradient_noise(q * 4.0f);
+        noise.patches = patches;
+        noise.grain = grain;
         tint = mk(1.0f + amount * (0.7f * patches + 0.3f * grain));
         tint *= mix3(mk(1.0f), mk(0.97f, 0.94f, 1.0f), gclamp(-patches, 0.0f, 1.0f) * gmin(1.0f, 5.0f * amount));
         wet = gclamp(0.8f + 0.4f * patches, 0.4f, 1.2f);
@@ -889,16 +921,63 @@ __device__ __noinline__ void apply_surface_texture(const PtArgs& A, f3 idx, Samp
     s.roughness = gclamp(s.roughness * rough, 0.02f, 1.0f);
     s.coat = gclamp(s.coat * wet, 0.0f, 1.0f);
 }
-// shading.glsl:328-342
-__device__ __noinline__ f3 bump_normal(const PtArgs& A, f3 idx, const Sample& s, f3 n) {
+// surface_height (shading.glsl:250-260) without lobules, 0.6 fbm(q) + 0.4 noise(4 q),
+// at p displaced by e along each axis. The displacement is a fiftieth of the
+// noise's cell times the octave, so the three points mostly lie in the cell of
+// p itself (q = p / scale): its eight corner vectors, most of a noise's work,
+// are hashed once for the three. The few points in another cell take the whole
+// noise afterwards, so that a warp does not run it at every point for one lane's
+// sake. A loop over the octaves keeps the code small. With p's own height from
+// its texture, 20 noises per shaded sample become 4, 4 sets of corners with 12
+// sums and about 2 more noises.
+__device__ __forceinline__ float octave_mul(int o) { return o == 0 ? 1.0f : o == 1 ? 2.03f : o == 2 ? 4.07f : 4.0f; }
+__device__ __forceinline__ float octave_add(int o) { return o == 1 ? 17.1f : o == 2 ? 31.7f : 0.0f; }
+__device__ __noinline__ f3 relief_heights(f3 p, float e, float scale, f3 q) {
+    const f3 a0 = (p + mk(e, 0.0f, 0.0f)) / scale, a1 = (p + mk(0.0f, e, 0.0f)) / scale,
+             a2 = (p + mk(0.0f, 0.0f, e)) / scale;
+    float n[12];
+    uint32_t crossed = 0;
+#pragma unroll 1
+    for (int o = 0; o < 4; o++) {
+        const float mul = octave_mul(o), add = octave_add(o);
+        const f3 c = q * mul + add;
+        const float flx = floorf(c.x), fly = floorf(c.y), flz = floorf(c.z);
+        const Lattice l = lattice_at((int)flx, (int)fly, (int)flz);
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const f3 x = (j == 0 ? a0 : j == 1 ? a1 : a2) * mul + add;
+            n[3 * o + j] = lattice_noise(l, mk(x.x - flx, x.y - fly, x.z - flz));
+            if (floorf(x.x) != flx || floorf(x.y) != fly || floorf(x.z) != flz) crossed |= 1u << (3 * o + j);
+        }
+    }
+    while (crossed) {
+        const int k = __ffs((int)crossed) - 1, o = k / 3, j = k - 3 * o;
+        crossed &= crossed - 1u;
+        n[k] = gradient_noise((j == 0 ? a0 : j == 1 ? a1 : a2) * octave_mul(o) + octave_add(o));
+    }
+    float h[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+        h[j] = two_products(0.4f, n[9 + j], 0.6f, (n[j] + 0.5f * n[3 + j] + 0.25f * n[6 + j]) / 1.75f);
+    return mk(h[0], h[1], h[2]);
+}
+// shading.glsl:328-342, `noise` from apply_surface_texture at the same point.
+__device__ __noinline__ f3 bump_normal(const PtArgs& A, const Sample& s, f3 n, const SurfaceNoise& noise) {
     if (!textured(A, s) || __ldg(&A.tab->surface[s.label].z) <= 0.0f || dot(n, n) < 0.5f) return n;
     float4 params = ldf4(&A.tab->surface[s.label]);
-    f3 p = index_to_world(A, idx);
+    f3 p = noise.p;
     float e = 0.02f * params.w;
-    float h = surface_height(p, params);
-    f3 g = mk(surface_height(p + mk(e, 0.0f, 0.0f), params) - h, surface_height(p + mk(0.0f, e, 0.0f), params) - h,
-              surface_height(p + mk(0.0f, 0.0f, e), params) - h) *
-           (params.z / e);
+    float h;
+    f3 moved;
+    if (params.x > 1.5f) {
+        h = lobule_height(p, params);
+        moved = mk(lobule_height(p + mk(e, 0.0f, 0.0f), params), lobule_height(p + mk(0.0f, e, 0.0f), params),
+                   lobule_height(p + mk(0.0f, 0.0f, e), params));
+    } else {
+        h = two_products(0.4f, noise.grain, 0.6f, noise.patches);
+        moved = relief_heights(p, e, params.w, p / params.w);
+    }
+    f3 g = (moved - h) * (params.z / e);
     return normalize(n - (g - dot(g, n) * n));
 }
 
@@ -1412,9 +1491,10 @@ __device__ __noinline__ void stage_shade(const PtArgs& A, const Consts& C, Path&
     f3 v = -P.dir;
     float surfaceness;
     surface_frame(A, V.idx, V.s, v, V.cap_plane, V.cut, 1.5f * C.step_mm, V.n, surfaceness);
-    apply_surface_texture(A, V.idx, V.s);
+    SurfaceNoise noise;
+    apply_surface_texture(A, V.idx, V.s, noise);
     V.surface_event = P.rng.rand() < surfaceness * (1.0f - V.s.subsurface) && dot(V.n, V.n) > 0.5f;
-    if (V.surface_event || P.bounce == 0u) V.n = bump_normal(A, V.idx, V.s, V.n);
+    if (V.surface_event || P.bounce == 0u) V.n = bump_normal(A, V.s, V.n, noise);
     if (P.bounce == 0u) {
         S.albedo.x += V.s.albedo.x; S.albedo.y += V.s.albedo.y; S.albedo.z += V.s.albedo.z;
         f3 nn = dot(V.n, v) < 0.0f ? -V.n : V.n;

@@ -1357,6 +1357,10 @@ static PtArgs pt_args(vv_renderer* r, const UHead& u) {
     return a;
 }
 
+// Words of a renderer's `work` buffer: the single-kernel tracers' work counter and
+// status, then the passes on the device (WfArgs::passes).
+enum { WORK_PASSES = 16 };
+
 // The wavefront state of pass `P` for `cap` paths in flight on stream `s`:
 // its records, queues, counters and later-flight bins over volume `v`
 // (allocated when the pass needs more than it has).
@@ -1473,6 +1477,7 @@ static cudaError_t run_pt(vv_renderer* r, vv_renderer::Pass& P, PtArgs& a, cudaS
     WfArgs w;
     cudaError_t ce = wf_state(P, cap, r->vol, s, w);
     if (ce != cudaSuccess) return ce;
+    w.passes = r->work.as<uint32_t>() + WORK_PASSES;
     return kernels_of(r).pt_wavefront(a, w, r->ctx->sms, s, launches);
 }
 
@@ -1984,7 +1989,9 @@ extern "C" vv_status vv_batch_create(vv_context* ctx, uint32_t passes, uint32_t 
         cudaError_t e = cudaStreamCreateWithFlags(&B.p.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&B.p.shown, cudaEventDisableTiming);
         if (e == cudaSuccess) e = B.p.counts.alloc(WF_COUNTERS * sizeof(uint32_t));
-        if (e == cudaSuccess) e = B.items.alloc(VV_BATCH_MAX * sizeof(uint32_t));
+        if (e == cudaSuccess) e = B.items.alloc((VV_BATCH_MAX + 1) * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemsetAsync(B.items.p, 0, B.items.n, B.p.stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(B.p.stream);  // passes on every stream count in pass 0's
         if (e == cudaSuccess) e = B.consts.alloc(VV_BATCH_MAX * WF_CONSTS_BYTES);
         if (e != cudaSuccess) {
             vv_batch_destroy(b);
@@ -2124,6 +2131,7 @@ extern "C" vv_status vv_batch_record(vv_batch* b, uint32_t n, vv_renderer* const
     WfArgs w;
     CK(wf_state(E.p, end, grid, s, w));
     w.items = E.items.as<uint32_t>();
+    w.passes = b->pass[0].items.as<uint32_t>() + VV_BATCH_MAX;
     w.consts = E.consts.p;
     int launches = 0;
     CK(fmt0::launch_pt_wavefront_batch(B, w, b->ctx->sms, s, &launches));

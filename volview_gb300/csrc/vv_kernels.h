@@ -99,7 +99,8 @@ enum {
     WF_STOP = 13,     // 0 while waves run; 1 + the queue index the finishing launch takes over
     WF_MAP = 14,      // light map shadow rays queued by the key light's shadow rays
     WF_TAKE_MAP = 15, // entries of the light map shadow queue taken so far
-    WF_COUNTERS = 16
+    WF_ALONE = 16,    // no other pass of this state's owner was on the device (shade looks, once per wave)
+    WF_COUNTERS = 17
 };
 struct WfArgs {
     uint32_t capacity;     // slots (and queue entries) allocated
@@ -129,6 +130,7 @@ struct WfArgs {
     int cell_shift;        // log2 of a cell's edge in voxels
     int cells_x, cells_y, cells_z;
     uint32_t bin_min;      // queues shorter than this are not ordered (the extend reads them as queued)
+    uint32_t* passes;      // passes of the state's owner (renderer or batch engine) on the device now
     // Batched passes only: each request's next work item (VV_BATCH_MAX words)
     // and its constants derived from the uniforms (VV_BATCH_MAX records of
     // WF_CONSTS_BYTES), written by the pass's first launch.

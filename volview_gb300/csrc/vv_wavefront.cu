@@ -387,6 +387,24 @@ __device__ void accumulate_items(const PtArgs& A, bool done, uint32_t item, cons
     atomicAdd(&A.normal[i], make_float4(v[8], v[9], v[10], v[11]));
 }
 
+constexpr uint32_t TAIL_ALONE = 2048u;
+// Lanes of each warp that take paths from a queue of n flights or shadow rays.
+// When no other pass of this state's owner is on the device, a short queue goes
+// to all warps of the launch, few lanes each: the divergent lanes of a warp take
+// turns, and a wave lasts as long as its slowest warp. Beside another pass the
+// same spreading takes issue slots that the other pass can use, so there every
+// warp takes 32. Measured (head/neck 1024^2): a frame alone 12.26 -> 11.07 ms and
+// overlapping frames 5.41 -> 5.43; spreading beside other passes too, 6.36. A
+// pass alone also leaves the waves earlier (TAIL_ALONE paths, 10.84 ms; 512, 1024
+// and 4096: 11.17, 11.07, 10.89). The count is looked at once per wave, between
+// its launches (WF_ALONE), so that all blocks of a launch see the same.
+__device__ __forceinline__ bool pass_alone(const WfArgs& W) { return W.counts[WF_ALONE] != 0u; }
+__device__ __forceinline__ bool takes_paths(const WfArgs& W, uint32_t n) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t lanes = pass_alone(W) ? (n + warps - 1u) / warps : 32u;
+    return (threadIdx.x & 31u) < lanes;
+}
+
 // Grid-stride loop over a queue with a warp-uniform bound, so that `push` sees
 // all 32 lanes.
 #define WF_FOR_EACH(n)                                                                          \
@@ -415,6 +433,7 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
         for (int k = 0; k < WF_COUNTERS; k++) W.counts[k] = 0;
         W.counts[WF_FIRST0] = slots;
         W.counts[WF_ITEMS] = slots;
+        W.counts[WF_ALONE] = atomicAdd(W.passes, 1u) == 0u;
     }
     if constexpr (IsBatch<X>::value) {
         if (blockIdx.x == 0 && threadIdx.x < B.n) {
@@ -466,7 +485,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
         // Every block reads the same counts (nothing changes them before this
         // launch ends), so all blocks decide alike.
         uint32_t live = W.counts[WF_FIRST0 + cur] + W.counts[cur];
-        if (live <= tail) {
+        if (live <= (pass_alone(W) ? max(tail, TAIL_ALONE) : tail)) {
             if (blockIdx.x == 0 && threadIdx.x == 0) W.counts[WF_STOP] = (uint32_t)cur + 1u;
             return;
         }
@@ -475,6 +494,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
     const uint32_t* queue = FIRST ? W.first[cur] : n < W.bin_min ? W.ext[cur] : W.sorted;
     uint32_t* taken = &W.counts[FIRST ? WF_TAKE_FIRST : WF_TAKE_EXT];
     const Consts C0 = kernel_consts(B);
+    const bool takes = takes_paths(W, n);
     uint32_t slot = 0, r = 0;
     f3 origin, dir, spectral;
     Rng rng;
@@ -482,7 +502,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
     Flight F;
     Vertex V;
     for (;;) {
-        const uint32_t k = take_item(taken, n, true);
+        const uint32_t k = take_item(taken, n, takes);
         int state = LANE_OUT, result = EXT_END;
         if (!__any_sync(0xffffffffu, k != ~0u)) break;
         if (k != ~0u) {
@@ -589,6 +609,7 @@ __global__ void __launch_bounds__(128, VV_SHADE_MIN_BLOCKS) k_wf_shade(const __g
         W.counts[WF_TAKE_EXT] = 0;
         W.counts[WF_TAKE_FIRST] = 0;
         W.counts[WF_ESC0 + (cur ^ 1)] = 0;  // finished by the previous wave's scatter
+        W.counts[WF_ALONE] = *(volatile uint32_t*)W.passes <= 1u;
     }
 }
 
@@ -623,12 +644,13 @@ template <bool MAP, class X>
 __global__ void __launch_bounds__(128, VV_SHADOW_MIN_BLOCKS) k_wf_shadow(const __grid_constant__ X B, const WfArgs W) {
     if (W.counts[WF_STOP] != 0u) return;
     const uint32_t n = W.counts[WF_SHADOW];
+    const bool takes = takes_paths(W, n);
     uint32_t slot = 0, r = 0;
     f3 origin;
     Rng rng;
     Shadow T;
     for (;;) {
-        const uint32_t k = take_item(&W.counts[WF_TAKE_SHADOW], n, true);
+        const uint32_t k = take_item(&W.counts[WF_TAKE_SHADOW], n, takes);
         if (!__any_sync(0xffffffffu, k != ~0u)) break;
         bool done = k != ~0u, to_map = false;
         if (done) {
@@ -674,12 +696,13 @@ __global__ void __launch_bounds__(128, VV_SHADOW_MIN_BLOCKS) k_wf_shadow_map(con
                                                                             const WfArgs W) {
     if (W.counts[WF_STOP] != 0u) return;
     const uint32_t n = W.counts[WF_MAP];
+    const bool takes = takes_paths(W, n);
     uint32_t slot = 0, r = 0;
     f3 origin;
     Rng rng;
     Shadow T;
     for (;;) {
-        const uint32_t k = take_item(&W.counts[WF_TAKE_MAP], n, true);
+        const uint32_t k = take_item(&W.counts[WF_TAKE_MAP], n, takes);
         if (!__any_sync(0xffffffffu, k != ~0u)) break;
         if (k != ~0u) {
             slot = W.map[k];
@@ -828,6 +851,7 @@ __global__ void __launch_bounds__(128, 4) k_wf_finish(const __grid_constant__ X 
     if (stop != 0u) cur = (int)stop - 1;  // else the waves ran out first: `cur` is the next wave's queue
     uint32_t n_first = W.counts[WF_FIRST0 + cur], n = n_first + W.counts[cur];
     const Consts C0 = kernel_consts(B);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicSub(W.passes, 1u);
     if ((threadIdx.x & 31u) != 0u) return;
     for (;;) {
         const uint32_t i = atomicAdd(&W.counts[WF_TAKE_EXT], 1u);  // zero: the last wave's shade cleared it

@@ -286,3 +286,59 @@ def test_tensor_core_convolution_long_runs(lib, cin, cout):
     close(got.astype(np.float64), want.astype(np.float64), 2e-3, 2e-3)
     failed = C.c_int(1)
     assert lib.vv_nn_tc_status(C.byref(failed), 1) == 0 and failed.value == 0
+
+
+# (n, h, w, cin, cout): row segments of 16, 32 and 64 pixels, runs that end inside
+# the image, channel tiles of 16, 32 and 48 with their remainders, one-row images.
+@pytest.mark.parametrize("shape", [(1, 1, 16, 16, 8), (2, 5, 48, 8, 24), (1, 7, 32, 40, 16), (1, 9, 64, 56, 56),
+                                   (1, 3, 192, 80, 104), (3, 31, 16, 176, 80), (1, 150, 64, 32, 32)])
+@pytest.mark.parametrize("shift", [0, 2])
+def test_weight_and_bias_gradients_at_tile_edges(lib, shape, shift):
+    """dw and db within 1e-3 of their largest magnitudes (the bar above), added
+    to what they held; tensors 4 bytes off a 16-byte boundary take the general
+    kernels."""
+    n, h, w, cin, cout = shape
+    rng = np.random.default_rng(sum(shape))
+    x, dy = rand_half(rng, (n, h, w, cin)), rand_half(rng, (n, h, w, cout))
+
+    def off(a):
+        t = torch.zeros(a.size + shift, dtype=torch.float16, device="cuda")
+        t[shift:] = dev(a, "half").reshape(-1)
+        return t[shift:]
+
+    xd, dd = off(x), off(dy)
+    dw, db = torch.full((cout, 3, 3, cin), 0.5, device="cuda"), torch.full((cout,), -1.0, device="cuda")
+    assert lib.vv_nn_conv3x3_wgrad(xd.data_ptr(), dd.data_ptr(), n, h, w, cin, cout, dw.data_ptr(), S) == 0
+    assert lib.vv_nn_bias_grad(dd.data_ptr(), n * h * w, cout, db.data_ptr(), S) == 0
+    pad = np.pad(x, ((0, 0), (1, 1), (1, 1), (0, 0)))
+    ref = np.stack([np.einsum("nhwo,nhwi->oi", dy, pad[:, t // 3:t // 3 + h, t % 3:t % 3 + w]) for t in range(9)], 1)
+    close(host(dw) - 0.5, ref.reshape(cout, 3, 3, cin), 1e-3)
+    close(host(db) + 1.0, dy.sum((0, 1, 2)), 1e-3)
+
+
+@pytest.mark.parametrize("c", [8, 24, 20])
+@pytest.mark.parametrize("n,h,w", [(1, 2, 2), (2, 6, 34)])
+def test_elementwise_gradients_at_vector_edges(lib, n, h, w, c):
+    """ReLU, addition, pooling, upsampling and split gradients, with channel
+    counts that are multiples of 8 (16 bytes per thread) and not: exact."""
+    rng = np.random.default_rng(n * h * w + c)
+    y, g, big = (rand_half(rng, (n, h, w, c)) for _ in range(3))
+    f16 = lambda a: a.astype(np.float32).astype(np.float16).astype(np.float64)  # noqa: E731
+    d = dev(g, "half")
+    assert lib.vv_nn_relu_backward(d.data_ptr(), dev(y, "half").data_ptr(), g.size, S) == 0
+    assert np.array_equal(host(d), np.where(y > 0, g, 0.0))
+    d = dev(g, "half")
+    assert lib.vv_nn_add(d.data_ptr(), dev(big, "half").data_ptr(), g.size, S) == 0
+    assert np.array_equal(host(d), f16(g + big))
+    out = torch.empty((n, 2 * h, 2 * w, c), dtype=torch.float16, device="cuda")
+    assert lib.vv_nn_avgpool2(dev(g, "half").data_ptr(), n, 2 * h, 2 * w, c, out.data_ptr(), 1, S) == 0
+    assert np.array_equal(host(out), f16(0.25 * g).repeat(2, 1).repeat(2, 2))
+    out = torch.empty((n, h // 2, w // 2, c), dtype=torch.float16, device="cuda")
+    assert lib.vv_nn_upsample2(dev(g, "half").data_ptr(), n, h // 2, w // 2, c, out.data_ptr(), 1, S) == 0
+    e = g.astype(np.float32)
+    assert np.array_equal(host(out), f16(((e[:, ::2, ::2] + e[:, ::2, 1::2]) + e[:, 1::2, ::2]) + e[:, 1::2, 1::2]))
+    for ca in (8, c - 8) if c > 8 else (4,):
+        a, b = (torch.empty((n, h, w, k), dtype=torch.float16, device="cuda") for k in (ca, c - ca))
+        gd = dev(g, "half")
+        assert lib.vv_nn_split(gd.data_ptr(), ca, c - ca, n * h * w, a.data_ptr(), b.data_ptr(), S) == 0
+        assert np.array_equal(host(a), g[..., :ca]) and np.array_equal(host(b), g[..., ca:])

@@ -197,6 +197,118 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad(const __half* __restrict_
     }
 }
 
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid) {  // zeros where not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0));
+}
+__device__ __forceinline__ void ldmatrix_t(uint32_t r[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+
+// The same gradient for 16-byte aligned tensors: a block of nine warps, one per
+// tap, takes 16 MT output and 16 CT input channels and walks `run` rows down a
+// segment of `seg` pixels. Row y's dy and the rows y - 1, y, y + 1 of x (one
+// pixel of halo) sit in shared memory, pixel-major as they lie, in rings of two
+// and four rows that cp.async fills one row ahead; both fragments come from
+// ldmatrix.trans (the reduction runs over pixels, the rows of both tiles), a
+// tap's x fragments `tap % 3` pixels further on. Row pitches are odd multiples
+// of 16 bytes, so the eight rows of a matrix fall in distinct banks. One FP32
+// add per weight and block at the end. Bound by shared memory and the legacy
+// tensor path; the kernel above (2-byte strided loads straight into fragments,
+// a chunk of 256 pixels per warp) took 1 718 us for the U-Net's 19 layers on
+// four 256 x 256 crops, this one 428 us (the largest, 80 -> 32: 332 -> 55).
+template <int MT, int CT>
+__global__ void __launch_bounds__(288, MT * CT > 6 ? 1 : 2) k_wgrad_tile(const __half* __restrict__ x, const __half* __restrict__ dy,
+                                                       int h, int w, int cin, int cout, int seg, int run,
+                                                       int co_tiles, float* __restrict__ dw) {
+    constexpr int XP = CT * 16 + 8, DP = MT * 16 + 8;  // row pitches, in halves
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t xs = smem_addr(smem), x_row = (uint32_t)(seg + 2) * XP * 2;
+    const uint32_t ds = xs + 4 * x_row, d_row = (uint32_t)seg * DP * 2;
+    const int tap = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int co0 = (int)(blockIdx.y % co_tiles) * MT * 16, ci0 = (int)(blockIdx.y / co_tiles) * CT * 16;
+    const int runs = (h + run - 1) / run, segs = w / seg;
+    const int column = (int)(blockIdx.x / runs), y0 = (int)(blockIdx.x % runs) * run;
+    const int img = column / segs, x0 = (column % segs) * seg;
+    const int rows = min(run, h - y0);
+    auto load_x = [&](int q) {  // image row y0 - 1 + q into slot q % 4
+        const int yy = y0 - 1 + q;
+        for (int i = threadIdx.x; i < (seg + 2) * CT * 2; i += 288) {
+            const int p = i / (CT * 2), c = i % (CT * 2), xx = x0 + p - 1;
+            const bool ok = yy >= 0 && yy < h && xx >= 0 && xx < w && ci0 + c * 8 < cin;
+            copy16(xs + (q & 3) * x_row + (p * XP + c * 8) * 2,
+                   ok ? x + (((long)img * h + yy) * w + xx) * cin + ci0 + c * 8 : x, ok);
+        }
+    };
+    auto load_d = [&](int q) {  // image row y0 + q into slot q % 2
+        for (int i = threadIdx.x; i < seg * MT * 2; i += 288) {
+            const int p = i / (MT * 2), c = i % (MT * 2);
+            const bool ok = co0 + c * 8 < cout;
+            copy16(ds + (q & 1) * d_row + (p * DP + c * 8) * 2,
+                   ok ? dy + (((long)img * h + y0 + q) * w + x0 + p) * cout + co0 + c * 8 : dy, ok);
+        }
+    };
+    float acc[MT][2 * CT][4];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int j = 0; j < 2 * CT; j++) acc[m][j][0] = acc[m][j][1] = acc[m][j][2] = acc[m][j][3] = 0.0f;
+    // This lane's row and column in a 16 x 16 group of four matrices: A (dy) in
+    // the order (pixels 0-7, channels 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15);
+    // B (x) (0-7, 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15).
+    const int r = lane & 7, id = lane >> 3;
+    const uint32_t a_off = (uint32_t)((((id >> 1) * 8 + r) * DP + (id & 1) * 8) * 2);
+    const uint32_t b_off = (uint32_t)((((id & 1) * 8 + r + tap % 3) * XP + (id >> 1) * 8) * 2);
+    load_x(0);
+    load_x(1);
+    load_x(2);
+    load_d(0);
+    asm volatile("cp.async.commit_group;");
+    for (int i = 0; i < rows; i++) {
+        if (i + 1 < rows) {
+            load_x(i + 3);
+            load_d(i + 1);
+        }
+        asm volatile("cp.async.commit_group;");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const uint32_t a_row = ds + (i & 1) * d_row + a_off, b_row = xs + ((i + tap / 3) & 3) * x_row + b_off;
+        for (int k = 0; k < seg; k += 16) {
+            uint32_t a[MT][4];
+#pragma unroll
+            for (int m = 0; m < MT; m++) ldmatrix_t(a[m], a_row + (k * DP + m * 16) * 2);
+#pragma unroll
+            for (int j = 0; j < CT; j++) {
+                uint32_t b[4];
+                ldmatrix_t(b, b_row + (k * XP + j * 16) * 2);
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    mma16816(acc[m][2 * j], a[m], b);
+                    mma16816(acc[m][2 * j + 1], a[m], b + 2);
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int j = 0; j < 2 * CT; j++) {
+            const int co = co0 + m * 16 + g, ci = ci0 + j * 8 + 2 * t;
+            if (ci >= cin) continue;
+            if (co < cout) {
+                atomicAdd(&dw[((long)co * 9 + tap) * cin + ci], acc[m][j][0]);
+                atomicAdd(&dw[((long)co * 9 + tap) * cin + ci + 1], acc[m][j][1]);
+            }
+            if (co + 8 < cout) {
+                atomicAdd(&dw[((long)(co + 8) * 9 + tap) * cin + ci], acc[m][j][2]);
+                atomicAdd(&dw[((long)(co + 8) * 9 + tap) * cin + ci + 1], acc[m][j][3]);
+            }
+        }
+}
+
 // db[c] += sum over pixels of dy[p][c].
 __global__ void k_bias_grad(const __half* __restrict__ dy, long pixels, int c, int chunk, float* __restrict__ db) {
     const int ch = threadIdx.x;
@@ -206,6 +318,119 @@ __global__ void k_bias_grad(const __half* __restrict__ dy, long pixels, int c, i
     float s = 0.0f;
     for (long p = first; p < last; p++) s += __half2float(dy[p * c + ch]);
     atomicAdd(&db[ch], s);
+}
+// k_bias_grad for 8 q channels and 16-byte aligned dy: a thread sums 8 channels
+// (16 bytes) of every (256 / q)-th pixel of the block's chunk, then the block
+// adds its threads' sums in shared memory, so that the reads are whole lines
+// and a channel takes one FP32 add per block. Measured on 262144 x 32: 12.7 us
+// before, 10.
+__global__ void __launch_bounds__(256) k_bias_grad_q(const uint4* __restrict__ dy, long pixels, int q, int chunk,
+                                                     float* __restrict__ db) {
+    extern __shared__ float part[];  // [256 / q][8 q]
+    const int lanes = 256 / q, k = threadIdx.x % q, first = threadIdx.x / q;
+    const long lo = (long)blockIdx.x * chunk, hi = lo + chunk < pixels ? lo + chunk : pixels;
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (first < lanes)
+        for (long p = lo + first; p < hi; p += lanes) {
+            const uint4 v = __ldg(dy + p * q + k);
+            const __half* e = (const __half*)&v;
+#pragma unroll
+            for (int j = 0; j < 8; j++) s[j] += __half2float(e[j]);
+        }
+    if (first < lanes)
+        for (int j = 0; j < 8; j++) part[(first * q + k) * 8 + j] = s[j];
+    __syncthreads();
+    for (int c = threadIdx.x; c < 8 * q; c += 256) {
+        float total = 0.0f;
+        for (int l = 0; l < lanes; l++) total += part[l * 8 * q + c];
+        atomicAdd(&db[c], total);
+    }
+}
+
+// The element-wise gradients, 8 halves (16 bytes) per thread where the tensors
+// are 16-byte aligned and their channels a multiple of 8: the same values, whole
+// lines instead of 2-byte accesses. On 262144 x 32, ReLU 23 -> 8.1 us; addition
+// 23 -> 7.3; splitting 80 channels 75 -> 20; upsampling 23 -> 7.3.
+__global__ void k_relu_backward_q(uint4* __restrict__ dy, const uint4* __restrict__ y, long count) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x) {
+        const uint4 v = __ldg(y + i);
+        uint4 d = dy[i];
+        const __half* e = (const __half*)&v;
+        __half* o = (__half*)&d;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (!(__half2float(e[j]) > 0.0f)) o[j] = __float2half_rn(0.0f);
+        dy[i] = d;
+    }
+}
+__global__ void k_add_q(uint4* __restrict__ y, const uint4* __restrict__ x, long count) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x) {
+        const uint4 v = __ldg(x + i);
+        uint4 s = y[i];
+        const __half* e = (const __half*)&v;
+        __half* o = (__half*)&s;
+#pragma unroll
+        for (int j = 0; j < 8; j++) o[j] = __float2half_rn(__half2float(o[j]) + __half2float(e[j]));
+        y[i] = s;
+    }
+}
+// Gradient of 2x2 pooling: a thread reads 8 channels of a pooled pixel and
+// writes its four pixels.
+__global__ void k_avgpool2_backward_q(const uint4* __restrict__ dy, int h, int w, int q, long total,
+                                      uint4* __restrict__ dx) {
+    const int ho = h / 2, wo = w / 2;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long p = i / q, row = p / wo;
+        const int k = (int)(i - p * q), xo = (int)(p - row * wo);
+        const long img = row / ho;
+        const int yo = (int)(row - img * ho);
+        const uint4 v = __ldg(dy + i);
+        const __half* e = (const __half*)&v;
+        uint4 r;
+        __half* o = (__half*)&r;
+#pragma unroll
+        for (int j = 0; j < 8; j++) o[j] = __float2half_rn(0.25f * __half2float(e[j]));
+        uint4* d = dx + ((img * h + 2 * yo) * w + 2 * xo) * q + k;
+        d[0] = r;
+        d[q] = r;
+        d[(long)w * q] = r;
+        d[(long)w * q + q] = r;
+    }
+}
+// Gradient of nearest 2x upsampling: the sums of 2x2 in k_upsample2_backward's order.
+__global__ void k_upsample2_backward_q(const uint4* __restrict__ dy, int h, int w, int q, long total,
+                                       uint4* __restrict__ dx) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long p = i / q, row = p / w;
+        const int k = (int)(i - p * q), xx = (int)(p - row * w);
+        const long img = row / h;
+        const int yy = (int)(row - img * h);
+        const uint4* b = dy + ((img * 2 * h + 2 * yy) * 2 * w + 2 * xx) * q + k;
+        const uint4 v00 = __ldg(b), v01 = __ldg(b + q), v10 = __ldg(b + 2L * w * q), v11 = __ldg(b + 2L * w * q + q);
+        const __half *e00 = (const __half*)&v00, *e01 = (const __half*)&v01, *e10 = (const __half*)&v10,
+                     *e11 = (const __half*)&v11;
+        uint4 r;
+        __half* o = (__half*)&r;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            o[j] = __float2half_rn(__half2float(e00[j]) + __half2float(e01[j]) + __half2float(e10[j]) +
+                                   __half2float(e11[j]));
+        dx[i] = r;
+    }
+}
+// The split of a concat's gradient (either part may be absent).
+__global__ void k_split_q(const uint4* __restrict__ dy, int qa, int qb, long total, uint4* __restrict__ da,
+                          uint4* __restrict__ db) {
+    const int q = qa + qb;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long p = i / q;
+        const int k = (int)(i - p * q);
+        if (k < qa) {
+            if (da) da[p * qa + k] = __ldg(dy + i);
+        } else if (db) {
+            db[p * qb + k - qa] = __ldg(dy + i);
+        }
+    }
 }
 
 __global__ void k_relu_backward(__half* __restrict__ dy, const __half* __restrict__ y, long count) {
@@ -371,6 +596,31 @@ __global__ void k_l1_loss(const __half* __restrict__ pred, int c, const float* _
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (3.0f * (float)pixels));
 }
 
+// k_l1_loss for c a multiple of 8 and 16-byte aligned pred and dpred: each
+// pixel's first 8 channels as one 16-byte read and write, zeros for the rest.
+__global__ void k_l1_loss_q(const uint4* __restrict__ pred, int q, const float* __restrict__ target, long pixels,
+                            float grad_scale, float* __restrict__ loss, uint4* __restrict__ dpred) {
+    long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    float s = 0.0f;
+    if (p < pixels) {
+        const float scale = grad_scale / (3.0f * (float)pixels);
+        const uint4 v = __ldg(pred + p * q);
+        const __half* e = (const __half*)&v;
+        __half g[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            float d = __half2float(e[k]) - target[p * 3 + k];
+            s += fabsf(d);
+            g[k] = __float2half_rn(d > 0.0f ? scale : (d < 0.0f ? -scale : 0.0f));
+        }
+        const __half zero = __float2half_rn(0.0f);
+        dpred[p * q] = make_uint4(pack(g[0], g[1]), pack(g[2], zero), 0u, 0u);
+        for (int k = 1; k < q; k++) dpred[p * q + k] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (3.0f * (float)pixels));
+}
+
 // Adam (Kingma and Ba) on FP32 master weights, with bias-corrected moments;
 // the FP16 copy the convolutions read is rewritten.
 __global__ void k_adam(float* __restrict__ w, __half* __restrict__ w16, const float* __restrict__ grad,
@@ -515,22 +765,70 @@ extern "C" vv_status vv_nn_flip_weights(const void* w, int cout, int cin, void* 
     return launched();
 }
 
+// 16-channel units of a weight-gradient tile over c channels: at most 3 (72
+// accumulators per lane at 3 x 3), the count that pads c least, the larger of two.
+static int wgrad_tile(int c) {
+    const int units = (c + 15) / 16;
+    if (units <= 3) return units;
+    const int pad3 = (units + 2) / 3 * 3, pad2 = (units + 1) / 2 * 2;
+    return pad3 <= pad2 ? 3 : 2;
+}
+template <int MT, int CT>
+static vv_status launch_wgrad(const __half* x, const __half* dy, int n, int h, int w, int cin, int cout, float* dw,
+                              cudaStream_t s) {
+    int sms = 152, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int seg = w % 64 == 0 ? 64 : w % 32 == 0 ? 32 : 16;
+    const int co_tiles = (cout + MT * 16 - 1) / (MT * 16), tiles = co_tiles * ((cin + CT * 16 - 1) / (CT * 16));
+    // Runs of rows so that about two blocks per SM cover the image.
+    const long columns = (long)n * (w / seg);
+    const long per_column = std::min<long>(h, std::max(1L, 2L * sms / (columns * tiles)));
+    const int run = (int)((h + per_column - 1) / per_column);
+    const long grid = columns * ((h + run - 1) / run);
+    const size_t smem = ((size_t)4 * (seg + 2) * (CT * 16 + 8) + (size_t)2 * seg * (MT * 16 + 8)) * 2;
+    if (grid > 0x7fffffffL) return VV_ERR_ARG;
+    k_wgrad_tile<MT, CT><<<dim3((unsigned)grid, tiles), 288, smem, s>>>(x, dy, h, w, cin, cout, seg, run, co_tiles, dw);
+    return launched();
+}
+
 extern "C" vv_status vv_nn_conv3x3_wgrad(const void* x, const void* dy, int n, int h, int w, int cin, int cout,
                                          float* dw, void* stream) {
     if (!x || !dy || !dw || n <= 0 || h <= 0 || w <= 0 || w % 16 || cin <= 0 || cin % 8 || cout <= 0 || cout % 8)
         return VV_ERR_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (aligned16(x) && aligned16(dy)) {
+        const __half *X = (const __half*)x, *D = (const __half*)dy;
+        switch (wgrad_tile(cout) * 4 + wgrad_tile(cin)) {
+            case 1 * 4 + 1: return launch_wgrad<1, 1>(X, D, n, h, w, cin, cout, dw, s);
+            case 1 * 4 + 2: return launch_wgrad<1, 2>(X, D, n, h, w, cin, cout, dw, s);
+            case 1 * 4 + 3: return launch_wgrad<1, 3>(X, D, n, h, w, cin, cout, dw, s);
+            case 2 * 4 + 1: return launch_wgrad<2, 1>(X, D, n, h, w, cin, cout, dw, s);
+            case 2 * 4 + 2: return launch_wgrad<2, 2>(X, D, n, h, w, cin, cout, dw, s);
+            case 2 * 4 + 3: return launch_wgrad<2, 3>(X, D, n, h, w, cin, cout, dw, s);
+            case 3 * 4 + 1: return launch_wgrad<3, 1>(X, D, n, h, w, cin, cout, dw, s);
+            case 3 * 4 + 2: return launch_wgrad<3, 2>(X, D, n, h, w, cin, cout, dw, s);
+            default: return launch_wgrad<3, 3>(X, D, n, h, w, cin, cout, dw, s);
+        }
+    }
     const int NT = 8;  // 64 input channels per warp
     const int chunk = 16;
     long tiles = (long)n * h * w / 16;
     dim3 grid(blocks(tiles, 4 * chunk), ((cout + 15) / 16) * ((cin + NT * 8 - 1) / (NT * 8)), 9);
-    k_conv3x3_wgrad<NT><<<grid, 128, 0, (cudaStream_t)stream>>>((const __half*)x, (const __half*)dy, n, h, w, cin,
-                                                                 cout, chunk, dw);
+    k_conv3x3_wgrad<NT><<<grid, 128, 0, s>>>((const __half*)x, (const __half*)dy, n, h, w, cin, cout, chunk, dw);
     return launched();
 }
 
 extern "C" vv_status vv_nn_bias_grad(const void* dy, long pixels, int c, float* db, void* stream) {
     if (!dy || !db || pixels <= 0 || c <= 0 || c > 1024) return VV_ERR_ARG;
     const int chunk = 256;
+    if (c % 8 == 0 && aligned16(dy)) {
+        const int q = c / 8;
+        // Up to 1024 pixels per block, fewer where that leaves SMs idle.
+        const int pixels_per_block = (int)std::min<long>(1024, std::max<long>(64, pixels / 304));
+        k_bias_grad_q<<<blocks(pixels, pixels_per_block), 256, (size_t)(256 / q) * 8 * q * sizeof(float),
+                        (cudaStream_t)stream>>>((const uint4*)dy, pixels, q, pixels_per_block, db);
+        return launched();
+    }
     k_bias_grad<<<blocks(pixels, chunk), c, 0, (cudaStream_t)stream>>>((const __half*)dy, pixels, c, chunk, db);
     return launched();
 }
@@ -538,6 +836,10 @@ extern "C" vv_status vv_nn_bias_grad(const void* dy, long pixels, int c, float* 
 extern "C" vv_status vv_nn_relu_backward(void* dy, const void* y, long count, void* stream) {
     if (!dy || !y || count < 0) return VV_ERR_ARG;
     if (count == 0) return VV_OK;
+    if (count % 8 == 0 && aligned16(dy) && aligned16(y)) {
+        k_relu_backward_q<<<grid_for(count / 8), 256, 0, (cudaStream_t)stream>>>((uint4*)dy, (const uint4*)y, count / 8);
+        return launched();
+    }
     k_relu_backward<<<blocks(count, 256), 256, 0, (cudaStream_t)stream>>>((__half*)dy, (const __half*)y, count);
     return launched();
 }
@@ -547,9 +849,13 @@ extern "C" vv_status vv_nn_avgpool2(const void* x, int n, int h, int w, int c, v
     if (!x || !y || n <= 0 || h <= 0 || w <= 0 || h % 2 || w % 2 || c <= 0) return VV_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     long out = backward ? (long)n * h * w * c : (long)n * (h / 2) * (w / 2) * c;
-    if (backward) {
+    const bool q = c % 8 == 0 && aligned16(x) && aligned16(y);
+    if (backward && q) {
+        const long total = (long)n * (h / 2) * (w / 2) * (c / 8);
+        k_avgpool2_backward_q<<<grid_for(total), 256, 0, s>>>((const uint4*)x, h, w, c / 8, total, (uint4*)y);
+    } else if (backward) {
         k_avgpool2_backward<<<blocks(out, 256), 256, 0, s>>>((const __half*)x, n, h, w, c, (__half*)y);
-    } else if (c % 8 == 0 && aligned16(x) && aligned16(y)) {
+    } else if (q) {
         k_avgpool2_q<<<grid_for(out / 8), 256, 0, s>>>((const uint4*)x, n, h, w, c / 8, (uint4*)y);
     } else {
         k_avgpool2<<<blocks(out, 256), 256, 0, s>>>((const __half*)x, n, h, w, c, (__half*)y);
@@ -562,7 +868,9 @@ extern "C" vv_status vv_nn_upsample2(const void* x, int n, int h, int w, int c, 
     if (!x || !y || n <= 0 || h <= 0 || w <= 0 || c <= 0) return VV_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     long out = backward ? (long)n * h * w * c : 4L * n * h * w * c;
-    if (backward) k_upsample2_backward<<<blocks(out, 256), 256, 0, s>>>((const __half*)x, n, h, w, c, (__half*)y);
+    if (backward && c % 8 == 0 && aligned16(x) && aligned16(y))
+        k_upsample2_backward_q<<<grid_for(out / 8), 256, 0, s>>>((const uint4*)x, h, w, c / 8, out / 8, (uint4*)y);
+    else if (backward) k_upsample2_backward<<<blocks(out, 256), 256, 0, s>>>((const __half*)x, n, h, w, c, (__half*)y);
     else k_upsample2<<<blocks(out, 256), 256, 0, s>>>((const __half*)x, n, h, w, c, (__half*)y);
     return launched();
 }
@@ -592,6 +900,11 @@ extern "C" vv_status vv_nn_upsample_concat(const void* a, int n, int h, int w, i
 extern "C" vv_status vv_nn_split(const void* dy, int ca, int cb, long pixels, void* da, void* db, void* stream) {
     if (!dy || ca <= 0 || cb <= 0 || pixels <= 0) return VV_ERR_ARG;
     long total = pixels * (ca + cb);
+    if (ca % 8 == 0 && cb % 8 == 0 && aligned16(dy) && aligned16(da) && aligned16(db)) {
+        k_split_q<<<grid_for(total / 8), 256, 0, (cudaStream_t)stream>>>((const uint4*)dy, ca / 8, cb / 8, total / 8,
+                                                                         (uint4*)da, (uint4*)db);
+        return launched();
+    }
     k_split<<<blocks(total, 256), 256, 0, (cudaStream_t)stream>>>((const __half*)dy, ca, cb, pixels, (__half*)da,
                                                                   (__half*)db);
     return launched();
@@ -608,6 +921,11 @@ extern "C" vv_status vv_nn_features(const float* accum, const float* albedo, con
 extern "C" vv_status vv_nn_l1_loss(const void* pred, int c, const float* target, long pixels, float grad_scale,
                                    float* loss, void* dpred, void* stream) {
     if (!pred || !target || !loss || !dpred || c < 3 || pixels <= 0 || !(grad_scale > 0.0f)) return VV_ERR_ARG;
+    if (c % 8 == 0 && aligned16(pred) && aligned16(dpred)) {
+        k_l1_loss_q<<<blocks(pixels, 256), 256, 0, (cudaStream_t)stream>>>((const uint4*)pred, c / 8, target, pixels,
+                                                                           grad_scale, loss, (uint4*)dpred);
+        return launched();
+    }
     k_l1_loss<<<blocks(pixels, 256), 256, 0, (cudaStream_t)stream>>>((const __half*)pred, c, target, pixels,
                                                                      grad_scale, loss, (__half*)dpred);
     return launched();
@@ -625,6 +943,10 @@ extern "C" vv_status vv_nn_adam(float* w, void* w16, const float* grad, float* m
 extern "C" vv_status vv_nn_add(void* y, const void* x, long count, void* stream) {
     if (!y || !x || count < 0) return VV_ERR_ARG;
     if (count == 0) return VV_OK;
+    if (count % 8 == 0 && aligned16(y) && aligned16(x)) {
+        k_add_q<<<grid_for(count / 8), 256, 0, (cudaStream_t)stream>>>((uint4*)y, (const uint4*)x, count / 8);
+        return launched();
+    }
     k_add<<<blocks(count, 256), 256, 0, (cudaStream_t)stream>>>((__half*)y, (const __half*)x, count);
     return launched();
 }

@@ -334,8 +334,8 @@ __device__ __noinline__ float density_cubic(const PtArgs& A, f3 p) {
     bspline_w(c.fz, wz);
     float acc = 0.0f;
     // Loops, not 64 unrolled taps: the flight kernels wait on instruction
-    // fetch, and the smaller code runs faster (349.7 -> 377.4 M path samples/s
-    // with both loops rolled and extinction_unclipped out of line).
+    // fetch, and the smaller code runs faster (rows unrolled: 672 M path
+    // samples/s against 670, but the ray marcher's frame 13.5 -> 14.3 ms).
 #pragma unroll 1
     for (int z = 0; z < 4; z++) {
         float az = 0.0f;
@@ -461,7 +461,7 @@ __device__ __forceinline__ bool label_solid(const PtArgs& A, uint32_t l, uint32_
 }
 
 // common.glsl:253-290
-__device__ __noinline__ Sample with_label(const PtArgs& A, Sample s, uint32_t label, uint32_t mode, bool ghost) {
+__device__ __forceinline__ Sample with_label(const PtArgs& A, Sample s, uint32_t label, uint32_t mode, bool ghost) {
     s.label = label;
     s.ghost = ghost;
     if (label == 0u) return s;
@@ -619,10 +619,16 @@ __device__ __forceinline__ Sample sample_point_unclipped(const PtArgs& A, f3 idx
 
 // common.glsl:395-404
 __device__ __noinline__ f3 mask_gradient(const PtArgs& A, f3 idx, int ch) {
-    f3 g;
-    g.x = mask_tri_ch(A, idx + mk(1.0f, 0.0f, 0.0f), ch) - mask_tri_ch(A, idx - mk(1.0f, 0.0f, 0.0f), ch);
-    g.y = mask_tri_ch(A, idx + mk(0.0f, 1.0f, 0.0f), ch) - mask_tri_ch(A, idx - mk(0.0f, 1.0f, 0.0f), ch);
-    g.z = mask_tri_ch(A, idx + mk(0.0f, 0.0f, 1.0f), ch) - mask_tri_ch(A, idx - mk(0.0f, 0.0f, 1.0f), ch);
+    // Three axes in a loop, not unrolled: the code of a ghost's shell in the flight
+    // kernels is as short as that (594 -> 635 M path samples/s; six lookups in a
+    // loop 612).
+    float d[3];
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {
+        const f3 e = mk(a == 0 ? 1.0f : 0.0f, a == 1 ? 1.0f : 0.0f, a == 2 ? 1.0f : 0.0f);
+        d[a] = mask_tri_ch(A, idx + e, ch) - mask_tri_ch(A, idx - e, ch);
+    }
+    f3 g = mk(d[0], d[1], d[2]);
     return mul_t(w2i3(A), 0.5f * g);
 }
 
@@ -757,7 +763,7 @@ __device__ __noinline__ float surface_frame(const PtArgs& A, f3 idx, const Sampl
 __device__ __forceinline__ bool measured(const PtArgs& A, const Sample& s) {
     return A.u.labels[0] >= 2.0f && s.label != 0u && !s.ghost && __ldg(&A.tab->optics[s.label].w) > 0.0f;
 }
-__device__ __noinline__ f3 tissue_sigma(const PtArgs& A, const Sample& s) {
+__device__ __forceinline__ f3 tissue_sigma(const PtArgs& A, const Sample& s) {
     float4 o = ldf4(&A.tab->optics[s.label]);
     f3 mu = mix3(mk(o.y), mk(o.x, o.y, o.z), A.u.env[3]);
     mu /= 1.0f - gclamp(A.u.env[2], 0.0f, 0.95f);
@@ -1219,18 +1225,35 @@ __device__ __noinline__ float bsdf_pdf(f3 n, f3 v, f3 l, const Sample& s) {
     return coat * ggx_pdf(n, v, l, cr * cr) + (1.0f - coat) * base;
 }
 
+// surface_frame's value (the extinction's scale) for a ghost, cap depth 0. Its
+// normal and surfaceness come from the ghost mask's gradient alone where that
+// has a length (skin keeps the density's normal); where the gradient is exactly
+// 0, inside a ghost, so is the value. The normals' volume is read, by the whole
+// function, for what remains.
+__device__ __forceinline__ float ghost_shell(const PtArgs& A, f3 idx, const Sample& s, f3 v, int cap_plane, float cut) {
+    if (s.label != SKIN_LABEL) {
+        f3 g = mask_gradient(A, idx, 1);
+        float g_len = len(g);
+        if (g_len == 0.0f) return 0.0f;
+        if (g_len > 1e-5f) {
+            f3 n = -g / g_len;
+            float edge_on = powf(1.0f - fabsf(dot(n, v)), 3.0f);
+            return gclamp(g_len * 4.0f, 0.0f, 1.0f) * mixf(A.u.labels[3], 1.0f, edge_on);
+        }
+    }
+    f3 n;
+    float surfaceness;
+    return surface_frame(A, idx, s, v, cap_plane, cut, 0.0f, n, surfaceness);
+}
+
 // pt.comp:277-292
 // extinction_at (pt.comp:277-292) after its clip test: the caller has found
 // `idx` inside the kept part (cut = clip_depth(idx) <= 0).
-__device__ __noinline__ float extinction_unclipped(const PtArgs& A, f3 idx, f3 dir, bool smooth, Sample& s, int& cap_plane,
+__device__ __forceinline__ float extinction_unclipped(const PtArgs& A, f3 idx, f3 dir, bool smooth, Sample& s, int& cap_plane,
                                       float& cut) {
     s = sample_labels<true>(A, idx, smooth && A.u.env[1] > 0.5f);
     if (s.extinction <= 0.0f) return 0.0f;
-    if (s.ghost) {
-        f3 n;
-        float surf;
-        return s.extinction * surface_frame(A, idx, s, -dir, cap_plane, cut, 0.0f, n, surf);
-    }
+    if (s.ghost) return s.extinction * ghost_shell(A, idx, s, -dir, cap_plane, cut);
     return s.extinction;
 }
 
@@ -1285,11 +1308,17 @@ __device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F,
     return clip_depth(A, origin + F.d_idx * F.tt, plane) <= 0.0f ? FF_SAMPLE : FF_CONTINUE;
 }
 // The rest of that iteration: the collision at F.tt, accepted (FF_HIT) or null.
-__device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
-                                         const Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
+// ff_fetch leaves its sample and returns the extinction there, a ghost's before
+// its shell's scale (ghost_shell); ff_collide decides on the extinction.
+__device__ __forceinline__ float ff_fetch(const PtArgs& A, f3 origin, bool smooth, const Flight& F, f3& idx, Sample& s,
+                                          int& cap_plane, float& cut) {
     idx = origin + F.d_idx * F.tt;
     cut = clip_depth(A, idx, cap_plane);
-    float ext = extinction_unclipped(A, idx, dir, smooth, s, cap_plane, cut);
+    s = sample_labels<true>(A, idx, smooth && A.u.env[1] > 0.5f);
+    return s.extinction;
+}
+__device__ __forceinline__ int ff_collide(const PtArgs& A, float ext, int hero, f3& spectral, const Flight& F,
+                                          const Sample& s, Rng& rng) {
     if (ext <= 0.0f) return FF_CONTINUE;
     f3 sigma = path_sigma(A, s, ext);
     float sh = comp(sigma, hero);
@@ -1299,6 +1328,12 @@ __device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, boo
     }
     spectral *= gmax(F.maj - sigma, 0.0f) / (F.maj - sh);
     return FF_CONTINUE;
+}
+__device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
+                                         const Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
+    float ext = ff_fetch(A, origin, smooth, F, idx, s, cap_plane, cut);
+    if (s.ghost && ext > 0.0f) ext *= ghost_shell(A, idx, s, -dir, cap_plane, cut);
+    return ff_collide(A, ext, hero, spectral, F, s, rng);
 }
 
 __device__ bool free_flight(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral, f3& idx,

@@ -458,7 +458,11 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
 // samples/s): phases with single-lane refill 327, refill at 8 ended lanes 476,
 // at 16 507-511, with all 32 ended 531-534. A refilled lane starts in the empty
 // bricks around the volume, or in another bin, and the other lanes wait through
-// its steps. VV_EXTEND_GATHER 12, 16, 20, 24, 28: 528, 532, 531, 530, 526.
+// its steps. With warps that coherent, code inline beats small code: ghosts'
+// shells without the normals volume 582, two advances per look at the warp 594,
+// mask gradients in a loop of three 635, labels, tissue and shell inline 682.
+// VV_EXTEND_GATHER 12, 16, 20, 28: 681, 678, 676, 667; a third phase that gathers
+// 1, 3, 8, 16 ghosts 653, 650, 643, 633; 10, 7, 6 blocks per SM 662, 661, 647.
 // Vertices go to shade; escapes and paths at the bounce limits go to this wave's
 // scatter kernel, which finishes them, so this kernel carries none of the
 // escape, accumulation or path-start code.
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
 #define VV_EXTEND_MIN_BLOCKS 8
 #endif
 #ifndef VV_EXTEND_GATHER
-#define VV_EXTEND_GATHER 20
+#define VV_EXTEND_GATHER 12
 #endif
 enum { EXT_END = 3 };
 enum { LANE_OUT, LANE_ADVANCE, LANE_SAMPLE };
@@ -531,7 +535,9 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
                 const unsigned advancing = __ballot_sync(0xffffffffu, state == LANE_ADVANCE);
                 sampling = __ballot_sync(0xffffffffu, state == LANE_SAMPLE);
                 if (!advancing || __popc(sampling) >= VV_EXTEND_GATHER) break;
-                if (state == LANE_ADVANCE) {
+#pragma unroll 1
+                for (int twice = 0; twice < 2; twice++) {  // one look at the warp per two advances
+                    if (state != LANE_ADVANCE) continue;
                     const int res = ff_advance(args_of(B, r), origin, F, rng);
                     if (res == FF_SAMPLE) state = LANE_SAMPLE;
                     if (res == FF_ESCAPE) {

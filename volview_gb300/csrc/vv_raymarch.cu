@@ -365,7 +365,11 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     const ShadowSweep w = shadow_sweep_of(A, sx, sy, sz, axis);
     const long at = ((long)p[2] * sy + p[1]) * sx + p[0];
     f3 here = mk((float)p[0], (float)p[1], (float)p[2]);
+    // The next slice's launch is prepared behind this one; it, too, waits for the
+    // slice before it (and so for all) past this point.
+    if (GIVEN) asm volatile("griddepcontrol.launch_dependents;");
     const float4 f = GIVEN ? __ldg(factors + at) : shadow_factors(A, w, here);
+    if (GIVEN) asm volatile("griddepcontrol.wait;" ::: "memory");
     f3 prev = here + w.l_idx * w.s;
     LightVol V{(const uint16_t*)vol, sx, sy, sz, 4};
     float4 back = lv_linear(V, (prev + 0.5f) / w.dims);
@@ -666,8 +670,22 @@ cudaError_t launch_shadow_sweep(const PtArgs& a, ushort4* vol, int sx, int sy, i
     int n = sd[axis];
     for (int i = 0; i < n; i++) {
         int slice = sign > 0 ? n - 1 - i : i;
-        if (factors) k_shadow_slice<true><<<g, 64, 0, s>>>(a, vol, factors, sx, sy, sz, axis, slice);
-        else k_shadow_slice<false><<<g, 64, 0, s>>>(a, vol, nullptr, sx, sy, sz, axis, slice);
+        if (factors) {
+            // Programmatic dependent launch: 6.7 -> 5.0 us per slice.
+            cudaLaunchConfig_t config = {};
+            config.gridDim = g;
+            config.blockDim = dim3(64);
+            config.stream = s;
+            cudaLaunchAttribute early[1];
+            early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            early[0].val.programmaticStreamSerializationAllowed = i > 0;  // the first follows the factors in full
+            config.attrs = early;
+            config.numAttrs = 1;
+            e = cudaLaunchKernelEx(&config, k_shadow_slice<true>, a, vol, (const float4*)factors, sx, sy, sz, axis, slice);
+            if (e != cudaSuccess) return e;
+        } else {
+            k_shadow_slice<false><<<g, 64, 0, s>>>(a, vol, nullptr, sx, sy, sz, axis, slice);
+        }
     }
     *launches += n;
     return cudaGetLastError();

@@ -13,6 +13,8 @@
 
 namespace vv {
 
+constexpr float MAX_EXTINCTION = 8.0f;  // pt.comp:34
+
 // --------------------------------------------------------------- float3 math
 struct f3 {
     float x, y, z;

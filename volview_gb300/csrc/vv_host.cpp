@@ -233,13 +233,14 @@ struct vv_renderer {
     float bucket[64];
     uint32_t majorants = VV_MAJORANTS_REFERENCE;  // VV_MAJORANTS_*: which bucket maxima
     // device volumes
-    DBuf density, normals, mask_a, mask_b, labels, majorant, lut, bucket_dev, tables, soft, work, exposure;
+    DBuf density, normals, mask_a, mask_b, labels, majorant, flight, lut, bucket_dev, tables, soft, work, exposure;
     int soft_dims[3] = {1, 1, 1};
     int soft_push[4] = {0, 0, 0, 0};
     bool has_labels = false;
     uint64_t generation = 0;
     bool have_mask_key = false, have_majorant_key = false;
     OpacityKey mask_key, majorant_key;
+    float flight_key[4] = {-1.0f, 0.0f, 0.0f, 0.0f};  // skipping, label modes, tissue and label extinction of `flight`
     // outputs
     uint32_t width = 0, height = 0;
     DBuf accum, albedo, normal, ping, pong, guide_nd, guide_alb, hdr, out, bloom[4];
@@ -737,6 +738,7 @@ extern "C" vv_status vv_renderer_create_ex(vv_context* ctx, const vv_volume* vol
     if ((e = r->density.alloc(elems * density_bytes(v.dfmt))) != cudaSuccess ||
         (e = r->normals.alloc(elems * sizeof(uint32_t))) != cudaSuccess ||
         (e = r->majorant.alloc((size_t)v.bx * v.by * v.bz * sizeof(float))) != cudaSuccess ||
+        (e = r->flight.alloc((size_t)v.bx * v.by * v.bz * sizeof(float))) != cudaSuccess ||
         (e = r->tables.alloc(sizeof(LabelTables))) != cudaSuccess ||
         (e = r->work.alloc(256)) != cudaSuccess || (e = r->exposure.alloc(sizeof(float))) != cudaSuccess) {
         hu.release();
@@ -810,6 +812,7 @@ extern "C" vv_status vv_renderer_create_view(vv_context* ctx, vv_renderer* base,
     root->views++;
     const long elems = vol_elems(r->vol);
     if ((e = r->majorant.alloc((size_t)r->vol.bx * r->vol.by * r->vol.bz * sizeof(float))) != cudaSuccess ||
+        (e = r->flight.alloc(r->majorant.n)) != cudaSuccess ||
         (e = r->tables.alloc(sizeof(LabelTables))) != cudaSuccess || (e = r->work.alloc(256)) != cudaSuccess ||
         (e = r->exposure.alloc(sizeof(float))) != cudaSuccess ||
         (r->has_labels && ((e = r->mask_a.alloc(elems * sizeof(uint32_t))) != cudaSuccess ||
@@ -842,7 +845,7 @@ extern "C" vv_status vv_renderer_destroy(vv_renderer* r) {
         if (P.stream) cudaStreamDestroy(P.stream);
     }
     if (r->prep_done) cudaEventDestroy(r->prep_done);
-    DBuf* all[] = {&r->density, &r->normals, &r->mask_a, &r->mask_b, &r->labels, &r->majorant, &r->env_rad,
+    DBuf* all[] = {&r->density, &r->normals, &r->mask_a, &r->mask_b, &r->labels, &r->majorant, &r->flight, &r->env_rad,
                    &r->env_table, &r->env_diffuse, &r->env_guide, &r->preint, &r->shadow_vol, &r->ao_vol, &r->lut,
                    &r->bucket_dev, &r->tables, &r->soft, &r->work, &r->exposure, &r->accum, &r->albedo,
                    &r->normal, &r->ping, &r->pong, &r->guide_nd, &r->guide_alb, &r->hdr, &r->out, &r->bloom[0], &r->bloom[1], &r->bloom[2],
@@ -1238,7 +1241,7 @@ extern "C" vv_status vv_query(vv_renderer* r, int* idle) {
 
 extern "C" vv_status vv_renderer_memory(const vv_renderer* r, uint64_t* bytes) {
     if (!r || !bytes) return fail(VV_ERR_ARG, "null argument");
-    const DBuf* all[] = {&r->density, &r->normals, &r->mask_a, &r->mask_b, &r->labels, &r->majorant, &r->lut,
+    const DBuf* all[] = {&r->density, &r->normals, &r->mask_a, &r->mask_b, &r->labels, &r->majorant, &r->flight, &r->lut,
                          &r->bucket_dev, &r->tables, &r->soft, &r->work, &r->exposure, &r->accum, &r->albedo,
                          &r->normal, &r->ping, &r->pong, &r->guide_nd, &r->guide_alb, &r->hdr, &r->out,
                          &r->bloom[0], &r->bloom[1], &r->bloom[2], &r->bloom[3], &r->preint, &r->shadow_vol,
@@ -1327,6 +1330,7 @@ static PtArgs pt_args(vv_renderer* r, const UHead& u) {
     a.normals = r->normals.as<uint32_t>();
     a.labels = r->labels.as<uint8_t>();
     a.majorant = r->majorant.as<float>();
+    a.flight = r->flight.as<float>();
     a.env_rad = r->env_rad.as<ushort4>();
     a.env_diffuse = r->env_diffuse.as<ushort4>();
     a.preint = r->preint.as<float4>();
@@ -1567,6 +1571,16 @@ static vv_status prepare_frame(vv_renderer* r, const vv_frame_params& p, uint64_
         r->launches += 1;
         r->majorant_key = key;
         r->have_majorant_key = true;
+        r->flight_key[0] = -1.0f;
+    }
+    // The flight majorants follow the bounds and the uniforms they depend on.
+    const float flight_key[4] = {u.path[3] != 0u ? 1.0f : 0.0f, u.labels[0] >= 2.0f ? 1.0f : 0.0f, u.tissue[0], u.labels[2]};
+    if (std::memcmp(flight_key, r->flight_key, sizeof(flight_key)) != 0) {
+        r->prep_work = true;
+        CK(launch_flight_majorant(r->majorant.as<float>(), r->vol.bx * r->vol.by * r->vol.bz, u.path[3] != 0u,
+                                  u.labels[0] >= 2.0f, u.tissue[0], u.labels[2], r->flight.as<float>(), st));
+        r->launches += 1;
+        std::memcpy(r->flight_key, flight_key, sizeof(flight_key));
     }
     if (p.path_tracing.enabled && r->accumulated == 0) {
         size_t bytes = (size_t)r->width * r->height * 16;

@@ -29,7 +29,8 @@ struct PtArgs {
     const uint32_t* mask;
     const uint32_t* normals;
     const uint8_t* labels;
-    const float* majorant;
+    const float* majorant;      // each brick's bound (majorant.comp)
+    const float* flight;        // its flight_majorant under these uniforms (k_flight_majorant)
     const float4* preint;       // cumulative transfer-function integrals, 4096 (ray marcher)
     const ushort4* env_diffuse; // light map's diffuse convolution, 32 x 16 RGBA16F (ray marcher)
     const ushort4* env_rad;     // light map radiance, RGBA16F, env_w x env_h (lighting.w == 2)
@@ -77,6 +78,9 @@ cudaError_t launch_normals(const void* d, uint32_t* out, const Vol& v, const m3&
 cudaError_t launch_masks(const MaskLaunch& L, cudaStream_t s, int* launches);
 cudaError_t launch_majorant(const void* d, const uint32_t* mask, const Vol& v, int mode, float label_ext,
                             const float* bucket, float* out, cudaStream_t s);
+// Each brick's flight_majorant (pt.comp:157-163) from its bound and the uniforms it depends on.
+cudaError_t launch_flight_majorant(const float* bound, int n, bool skip, bool labelled, float tissue, float label_ext,
+                                   float* out, cudaStream_t s);
 cudaError_t launch_unbrick(const void* src, void* dst, const Vol& v, int elem, cudaStream_t s);
 cudaError_t launch_brick_u8(const uint8_t* src, uint8_t* dst, const Vol& v, cudaStream_t s);
 

@@ -57,7 +57,6 @@ namespace {
 
 
 constexpr float PI = 3.14159265358979f;
-constexpr float MAX_EXTINCTION = 8.0f;       // pt.comp:34
 constexpr uint32_t MAX_VOLUME_EVENTS = 32u;  // pt.comp:112
 constexpr float BONE_DENSITY = (300.0f + 1024.0f) / 4095.0f;
 constexpr uint32_t SKIN_LABEL = 255u;
@@ -1164,15 +1163,11 @@ __device__ __forceinline__ f3 event_albedo(const PtArgs& A, const Sample& s) {
     f3 reduced = single_scattering_albedo(s.albedo);
     return measured(A, s) ? 1.0f - (1.0f - reduced) * (1.0f - gclamp(A.u.env[2], 0.0f, 0.95f)) : reduced;
 }
-// flight_majorant (pt.comp:157-163) of brick `b` (brick_index).
+// flight_majorant (pt.comp:157-163) of brick `b` (brick_index), from the grid
+// prepared for the frame's uniforms.
 __device__ __forceinline__ float flight_majorant_of(const PtArgs& A, int b) {
-    float m = 1e30f;
-    if (A.u.path[3] != 0u) {
-        count(A, COUNT_MAJORANT);
-        m = __ldg(A.majorant + b);
-    }
-    if (m > 0.0f && A.u.labels[0] >= 2.0f) m = gmax(m, A.u.tissue[0]);
-    return gmin(m, gmax(MAX_EXTINCTION, gmax(A.u.labels[2], A.u.tissue[0])));
+    if (A.u.path[3] != 0u) count(A, COUNT_MAJORANT);
+    return __ldg(A.flight + b);
 }
 __device__ __forceinline__ float phase_hg(const PtArgs& A, float cos_t) {
     float g = A.u.env[2];
@@ -1264,8 +1259,7 @@ struct Flight {
     f3 d_idx, inv_d;
     float tt, t_end;
     int iter;
-    int brick;    // brick whose flight majorant `maj` holds (-1: none yet)
-    float maj;
+    float maj;    // flight majorant at tt
 };
 enum { FF_CONTINUE = 0, FF_HIT = 1, FF_ESCAPE = 2, FF_SAMPLE = 4 };
 
@@ -1276,22 +1270,19 @@ __device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Fli
     F.tt = tr.x;
     F.t_end = tr.y;
     F.iter = 0;
-    F.brick = -1;
 }
 
 // One iteration of pt.comp:307-333 up to the voxel fetch. FF_CONTINUE: an
 // empty brick, a sample beyond the brick exit, or a tentative collision in the
 // clipped part (extinction_at returns 0 there before any fetch); FF_SAMPLE: a
 // tentative collision at F.tt that needs the volume (ff_sample); FF_ESCAPE.
-// The majorant of the brick the ray is in is fetched once per brick.
+// The majorant is fetched at every advance: from the prepared grid that is
+// cheaper than looking whether the brick has changed (711 M path samples/s against
+// 705; 685 when every fetch applied the uniforms).
 __device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F, Rng& rng) {
     if (!(F.iter < 4096 && F.tt < F.t_end)) return FF_ESCAPE;
     f3 p = origin + F.d_idx * F.tt;
-    int b = brick_index(A, p);
-    if (b != F.brick) {
-        F.brick = b;
-        F.maj = flight_majorant_of(A, b);
-    }
+    F.maj = flight_majorant_of(A, brick_index(A, p));
     F.iter++;
     float exit = F.tt + brick_exit(p, F.inv_d, far_planes(F.inv_d)) + 1e-3f;
     if (F.maj <= 0.0f) {

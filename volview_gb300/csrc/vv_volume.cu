@@ -515,6 +515,18 @@ __global__ void __launch_bounds__(256) k_majorant(const void* __restrict__ d, co
     out[b] = bound;
 }
 
+// flight_majorant (pt.comp:157-163) of every brick, for the tracer's uniforms:
+// the brick's bound, or none without empty-space skipping; at least the tissue's
+// where labels are drawn alone; at most the largest of the three caps.
+__global__ void __launch_bounds__(256) k_flight_majorant(const float* __restrict__ bound, int n, int skip, int labelled,
+                                                         float tissue, float label_ext, float* __restrict__ out) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= n) return;
+    float m = skip ? bound[b] : 1e30f;
+    if (m > 0.0f && labelled) m = gmax(m, tissue);
+    out[b] = gmin(m, gmax(MAX_EXTINCTION, gmax(label_ext, tissue)));
+}
+
 // Bricked -> x-fastest copy of `elem`-byte elements.
 __global__ void k_unbrick(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, Vol v, int elem) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -610,6 +622,11 @@ cudaError_t launch_majorant(const void* d, const uint32_t* mask, const Vol& v, i
     const unsigned nb = blocks_for((long)v.bx * v.by * v.bz, 8);  // a warp per brick
     if (v.dfmt == DF_FP32) k_majorant<true><<<nb, 256, 0, s>>>(d, mask, v, mode, label_ext, bucket, out);
     else k_majorant<false><<<nb, 256, 0, s>>>(d, mask, v, mode, label_ext, bucket, out);
+    return cudaGetLastError();
+}
+cudaError_t launch_flight_majorant(const float* bound, int n, bool skip, bool labelled, float tissue, float label_ext,
+                                   float* out, cudaStream_t s) {
+    k_flight_majorant<<<blocks_for(n, 256), 256, 0, s>>>(bound, n, skip, labelled, tissue, label_ext, out);
     return cudaGetLastError();
 }
 cudaError_t launch_unbrick(const void* src, void* dst, const Vol& v, int elem, cudaStream_t s) {

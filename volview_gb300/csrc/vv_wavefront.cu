@@ -480,6 +480,7 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
 #define VV_EXTEND_GATHER 12
 #endif
 enum { EXT_END = 3 };
+constexpr uint32_t ESC_BACKGROUND = 0x80000000u;  // slots are below 2^31 (the host's limit on items)
 enum { LANE_OUT, LANE_ADVANCE, LANE_SAMPLE };
 // FIRST: the first-flight queue (bounce 0: cubic B-spline density along the
 // flight), otherwise later flights (trilinear); each kernel carries only its
@@ -565,7 +566,11 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
                 }
             }
         }
-        if (k != ~0u) {
+        // A first flight that leaves the volume ends its item when the frame has
+        // one sample per pixel: background, whose sums are known. Scatter needs
+        // the item alone, so nothing is written for it (ESC_BACKGROUND marks it).
+        const bool background = FIRST && k != ~0u && result == FF_ESCAPE && args_of(B, r).u.path[2] == 1u;
+        if (k != ~0u && !background) {
             if (result != EXT_END) {  // free flight changed the spectral ratios
                 float4* q = rec(W.path, slot, PATH_N);
                 float4 d = q[3];
@@ -583,7 +588,8 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
             }
         }
         push(W.shade, &W.counts[WF_SHADE], slot, k != ~0u && result == FF_HIT);
-        push(W.esc[cur], &W.counts[WF_ESC0 + cur], slot, k != ~0u && result != FF_HIT);
+        push(W.esc[cur], &W.counts[WF_ESC0 + cur], background ? slot | ESC_BACKGROUND : slot,
+             k != ~0u && result != FF_HIT);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) W.counts[WF_SCATTER] = 0;
 }
@@ -757,14 +763,22 @@ __global__ void __launch_bounds__(128, VV_SCATTER_MIN_BLOCKS) k_wf_scatter(const
         uint32_t i = base_ + (threadIdx.x & 31u);
         bool valid = i < n;
         bool ended = i >= n_scatter;
-        uint32_t slot = valid ? (ended ? W.esc[cur][i - n_scatter] : W.scatter[i]) : 0u;
+        const uint32_t entry = valid ? (ended ? W.esc[cur][i - n_scatter] : W.scatter[i]) : 0u;
+        const bool background = (entry & ESC_BACKGROUND) != 0u;
+        const uint32_t slot = entry & ~ESC_BACKGROUND;
         const uint32_t r = request_of(B, slot);
         const PtArgs& A = args_of(B, r);
         const Consts& C = consts_of(B, W, r, C0);
         bool to_ext = false, to_first = false, done = false;
         uint32_t item = 0, key = 0;
         PixelSums S;
-        if (valid) {
+        if (valid && background) {
+            // stage_escape and finish_path of a path without a vertex: coverage, a
+            // white albedo, the far depth (pt.comp:434-439); its item is done.
+            item = ubits(rec(W.acc, slot, ACC_N)[0].w);
+            S = {mk(0.0f), 1.0f, make_float4(1.0f, 1.0f, 1.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 1e4f)};
+            done = true;
+        } else if (valid) {
             Path P;
             uint32_t sample;
             load_path(W, slot, P, sample);

@@ -1443,12 +1443,14 @@ static cudaError_t wf_state(vv_renderer::Pass& P, size_t cap, const Vol& v, cuda
         w.cells_x = cx;
         w.cells_y = cy;
         w.cells_z = cz;
-        // Queues of fewer than 16384 later flights go unordered (the late
-        // waves, whose chains of launches the ordering lengthened): 392.7 ->
-        // 394.2 M path samples/s, one vv_record per frame 7.08 -> 6.90 ms
-        // (65536: 393.0 and 7.07; 262144: 392.2 and 7.03).
+        // Queues of at most 65536 later flights go unordered, and a pass that
+        // has no more path slots queues no ordering launches at all: in the
+        // late waves the three launches cost the chain more than the order
+        // gives. Against a line at 16384: 1024^2 frame 8.21 -> 8.06 ms, a
+        // 256^2 frame 3.20 -> 3.07, 16-frame passes alone 29.4 -> 29.0 and
+        // overlapped 22.9 -> 23.0 (within the runs' spread); 131072 the same.
         const char* e = std::getenv("VV_WF_BIN_MIN");
-        w.bin_min = e ? (uint32_t)std::max(0, std::atoi(e)) : 16384u;
+        w.bin_min = e ? (uint32_t)std::max(0, std::atoi(e)) : 65537u;
     }
     return cudaSuccess;
 }

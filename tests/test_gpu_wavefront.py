@@ -1,0 +1,137 @@
+"""How the wavefront tracer schedules its paths changes none of them (GPU): the
+ordering of the later flights, a pass alone (short queues spread over the chip)
+or beside another renderer's, slots refilled or not, background paths that end
+with their item, and the prepared grid of flight majorants.
+
+A pass of one frame per pixel stores its sums without atomics, so those images
+are compared bit by bit. Frames accumulated by one pass are added with float
+atomics in an order the device decides: N positive FP32 terms in any order
+differ by at most about N * 2^-23 relative, so 1e-5 holds for the sums of up
+to 40 frames here."""
+import numpy as np
+import pytest
+
+from volview_gb300 import abi, scene
+from volview_gb300 import renderer as R
+
+pytestmark = pytest.mark.gpu
+
+
+def _renderer(cfg, ctx, env=None):
+    r = R.Renderer(ctx, cfg["volume"], cfg["tf"])
+    r.set_labels(cfg["labels_vol"], abi.soft_struct(cfg["soft"]))
+    if env is not None:
+        r.set_environment_map(abi.env_struct(env))
+    return r
+
+
+def _params(cfg, r, near=0.5):
+    p = scene.frame_params_for(cfg, list(r.center), r.diagonal, clip_sagittal=True)
+    p.camera.distance = abi.f32(p.camera.distance * near)
+    p.path_tracing.denoiser = abi.DENOISE_OFF
+    return p
+
+
+def _frame(r, p):
+    r.reset_view()
+    r.record(1, p)
+    return r.read_accumulation()
+
+
+@pytest.mark.parametrize("light", ["studio", "map"])
+@pytest.mark.parametrize("size", [(1, 1), (37, 21), (131, 77)])
+def test_order_and_company_change_no_path(small_cfg, gpu_ctx, monkeypatch, size, light):
+    """131 x 77 paths run through the waves and then the finishing launch, the
+    smaller images through the finishing launch alone."""
+    cfg = small_cfg
+    r = _renderer(cfg, gpu_ctx, scene.synthetic_light_map() if light == "map" else None)
+    ctx = R.Context(0)
+    other = _renderer(cfg, ctx)
+    try:
+        p = _params(cfg, r)
+        if light == "map":
+            p.lighting.environment = abi.ENV_MAP
+        r.resize(*size)
+        other.resize(96, 64)
+        q = _params(cfg, other)
+        images = []
+        for bin_min, company in ((None, False), ("0", False), (None, True), ("0", True)):
+            if bin_min is None:
+                monkeypatch.delenv("VV_WF_BIN_MIN", raising=False)
+            else:
+                monkeypatch.setenv("VV_WF_BIN_MIN", bin_min)
+            if company:
+                other.reset_view()
+                other.record_frames(1, 32, q)
+            images.append(_frame(r, p))
+            other.synchronize()
+        assert size == (1, 1) or np.any(images[0][0][..., :3])
+        for image in images[1:]:
+            for a, b in zip(image, images[0]):
+                assert np.array_equal(a, b)
+    finally:
+        r.destroy()
+        other.destroy()
+        ctx.destroy()
+
+
+@pytest.mark.parametrize("slot_frames", [16, 2])
+@pytest.mark.parametrize("near", [0.4, 3.0])
+def test_frames_of_one_pass_sum_to_single_frames(small_cfg, gpu_ctx, near, slot_frames):
+    """Eight frames in one pass (with slots for all of them, and refilled from
+    two frames' worth) against eight single frames, close up and at a distance
+    where most paths leave the volume at once."""
+    cfg = small_cfg
+    r = _renderer(cfg, gpu_ctx)
+    try:
+        p = _params(cfg, r, near)
+        r.resize(83, 59)
+        for f in range(8):
+            r.record(f + 1, p)
+        single = r.read_accumulation()
+        r.reset_view()
+        r.set_pass_budget(2, slot_frames)
+        r.record_frames(1, 8, p)
+        for a, b in zip(r.read_accumulation(), single):
+            assert np.all(np.abs(a - b) <= 1e-5 * np.abs(b) + 1e-6)
+    finally:
+        r.destroy()
+
+
+def test_flight_majorants_follow_their_inputs(small_cfg, gpu_ctx):
+    """A renderer whose parameters change between frames gives the images of
+    fresh renderers: the flight majorants follow the skipping of empty space,
+    the label mode, the label extinction and the tissues' anisotropy."""
+    cfg = small_cfg
+    kept = _renderer(cfg, gpu_ctx)
+    try:
+        kept.resize(61, 43)
+
+        def base():
+            return _params(cfg, kept)
+
+        def skipping(p):
+            p.skip_empty_space = 0
+
+        def mode(p):
+            p.labels.mode = abi.LABEL_TINT
+
+        def extinction(p):
+            p.labels.extinction = abi.f32(p.labels.extinction * 0.5)
+
+        def anisotropy(p):
+            p.lighting.anisotropy = abi.f32(0.9)
+
+        for change in (lambda p: None, skipping, extinction, anisotropy, mode, skipping, lambda p: None):
+            p = base()
+            change(p)
+            image = _frame(kept, p)
+            fresh = _renderer(cfg, gpu_ctx)
+            try:
+                fresh.resize(61, 43)
+                for a, b in zip(image, _frame(fresh, p)):
+                    assert np.array_equal(a, b)
+            finally:
+                fresh.destroy()
+    finally:
+        kept.destroy()

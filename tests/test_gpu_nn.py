@@ -288,6 +288,50 @@ def test_tensor_core_convolution_long_runs(lib, cin, cout):
     assert lib.vv_nn_tc_status(C.byref(failed), 1) == 0 and failed.value == 0
 
 
+# Output channels in groups: 2 of 32 beside three rows, 5 of 16 beside three, 2 of 64
+# (the last of 48), 2 of 80 (the last of 64), 2 of 96 (the last of 80); one-row images.
+@pytest.mark.parametrize("shape", [(1, 5, 256, 144, 64), (1, 9, 128, 176, 80), (2, 3, 128, 48, 112),
+                                   (1, 1, 128, 64, 144), (1, 4, 256, 80, 176)])
+def test_tensor_core_convolution_in_channel_groups(lib, shape):
+    """Shapes whose weights do not fit in shared memory at once, against the
+    reference at the convolution tolerance."""
+    import ctypes as C
+    n, h, w, cin, cout = shape
+    rng = np.random.default_rng(cin + cout)
+    x, wt = rand_half(rng, (n, h, w, cin)), rand_half(rng, (cout, 3, 3, cin), 0.1)
+    b = rng.standard_normal(cout).astype(np.float32)
+    X, W, B = dev(x, "half"), dev(wt, "half"), dev(b)
+    Y = torch.empty((n, h, w, cout), dtype=torch.float16, device="cuda")
+    for relu, bias in ((0, b), (1, b), (1, None)):
+        assert lib.vv_nn_conv3x3(X.data_ptr(), n, h, w, cin, W.data_ptr(), B.data_ptr() if bias is not None else None,
+                                 cout, relu, Y.data_ptr(), S) == 0
+        close(host(Y), N.conv3x3(x, wt, np.zeros(cout, np.float32) if bias is None else b, bool(relu)), 2e-3, 2e-3)
+    failed = C.c_int(1)
+    assert lib.vv_nn_tc_status(C.byref(failed), 1) == 0 and failed.value == 0
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 32), (32, 8), (64, 64), (96, 64), (144, 64)])
+def test_tensor_core_convolution_wraps_its_ring(lib, cin, cout):
+    """Many images make every CTA's run longer than its ring of row slots (eight
+    slots, four with 96 -> 64 channels, three with 144 -> 64), against PyTorch's
+    FP64 convolution at the convolution tolerance."""
+    import ctypes as C
+    torch.manual_seed(cin + cout)
+    n, h, w = 304, 19, 128
+    x = (torch.randn((n, h, w, cin), device="cuda") * 0.5).half()
+    wt = (torch.randn((cout, 3, 3, cin), device="cuda") * 0.1).half()
+    y = torch.empty((n, h, w, cout), dtype=torch.float16, device="cuda")
+    assert lib.vv_nn_conv3x3(x.data_ptr(), n, h, w, cin, wt.data_ptr(), None, cout, 1, y.data_ptr(), S) == 0
+    for part in range(0, n, 76):
+        ref = torch.nn.functional.conv2d(x[part:part + 76].double().permute(0, 3, 1, 2),
+                                         wt.double().permute(0, 3, 1, 2), padding=1)
+        ref = torch.relu(ref).permute(0, 2, 3, 1)
+        torch.cuda.synchronize()
+        close(y[part:part + 76].double().cpu().numpy(), ref.cpu().numpy(), 2e-3, 2e-3)
+    failed = C.c_int(1)
+    assert lib.vv_nn_tc_status(C.byref(failed), 1) == 0 and failed.value == 0
+
+
 # (n, h, w, cin, cout): row segments of 16, 32 and 64 pixels, runs that end inside
 # the image, channel tiles of 16, 32 and 48 with their remainders, one-row images.
 @pytest.mark.parametrize("shape", [(1, 1, 16, 16, 8), (2, 5, 48, 8, 24), (1, 7, 32, 40, 16), (1, 9, 64, 56, 56),

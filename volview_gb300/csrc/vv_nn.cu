@@ -24,7 +24,7 @@ namespace nn {
 
 // vv_nn_tc.cu: the tcgen05 convolution; false when the shape is not one it takes.
 bool conv3x3_tc(const __half* x, int n, int h, int w, int cin, const __half* wt, const float* bias, int cout,
-                int relu, __half* y, cudaStream_t s, cudaError_t* err);
+                int relu, __half* y, cudaStream_t s, bool grouped, cudaError_t* err);
 
 __device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], const uint32_t b[2]) {
     asm volatile(
@@ -719,10 +719,10 @@ extern "C" vv_status vv_nn_conv3x3(const void* x, int n, int h, int w, int cin, 
         case 8: case 16: case 32: case 48: case 64: case 80: case 96: case 112: case 144: case 176: break;
         default: return VV_ERR_ARG;
     }
-    // Widths that are multiples of 128 with the weights and two segments'
-    // input rows in shared memory run on tcgen05 (vv_nn_tc.cu); the rest here.
+    // Widths that are multiples of 128 run on tcgen05 (vv_nn_tc.cu), their
+    // channels in groups where the weights do not fit at once; the rest here.
     cudaError_t te = cudaSuccess;
-    if (conv3x3_tc((const __half*)x, n, h, w, cin, (const __half*)weights, bias, cout, relu, (__half*)y, s, &te))
+    if (conv3x3_tc((const __half*)x, n, h, w, cin, (const __half*)weights, bias, cout, relu, (__half*)y, s, false, &te))
         return te == cudaSuccess ? VV_OK : VV_ERR_CUDA;
     const unsigned g = blocks((long)n * h * w / 16, CONV_WARPS);
     const __half* X = (const __half*)x;
@@ -747,6 +747,8 @@ extern "C" vv_status vv_nn_conv3x3(const void* x, int n, int h, int w, int cin, 
     }
     const size_t smem = (size_t)nt * 8 * (cin + 8) * sizeof(__half);
     if (smem > 48 * 1024) return VV_ERR_ARG;  // one tap's weights staged in shared memory
+    if (conv3x3_tc((const __half*)x, n, h, w, cin, (const __half*)weights, bias, cout, relu, (__half*)y, s, true, &te))
+        return te == cudaSuccess ? VV_OK : VV_ERR_CUDA;
     const dim3 grid(g, tiles / nt);
     switch (nt) {
         case 1: k_conv3x3<1><<<grid, CONV_WARPS * 32, smem, s>>>(X, n, h, w, cin, W, bias, relu, Y, cout); break;

@@ -9,20 +9,20 @@
 // core matrices, the 8-row groups of one 16-byte K slice 128 bytes apart (the
 // stride byte offset), consecutive K slices LBO bytes apart.
 //
-// A CTA keeps all nine taps' weights in shared memory and walks down a run
-// of rows of one column of segments (the same 128 pixels of consecutive
-// rows). Its input rows, each with its one-pixel halo (130 pixels), sit in a
-// ring of four row slots: a segment uses three (rows y-1, y, y+1) and the
-// fourth takes the next row, so every input row is copied once per run. TMA
-// copies a row as boxes of 8 channels x 130 pixels, one per 16-byte channel
-// slice, zero-filled outside the image (same padding); such a box is one K
-// slice of the layout above. Tap (dy, dx)'s A operand is row y+dy-1's slices
-// starting dx pixels in: the descriptor's start address moves by 16 bytes per
-// pixel. Roles:
-//   warp 4 (one lane): waits for a segment's three rows, issues its
+// A CTA keeps all nine taps' weights of its output channels in shared memory
+// and walks down a run of rows of one column of segments (the same 128 pixels
+// of consecutive rows). Its input rows, each with its one-pixel halo (130
+// pixels), sit in a ring of row slots: a segment uses three (rows y-1, y, y+1)
+// and the others take the rows ahead, so every input row is copied once per
+// run. TMA copies a row as one box of its 16-byte channel slices x 130 pixels,
+// zero-filled outside the image (same padding); each slice is one K slice of
+// the layout above. Tap (dy, dx)'s A operand is row y+dy-1's slices starting
+// dx pixels in: the descriptor's start address moves by 16 bytes per pixel.
+// Roles:
+//   warp 4 (its elected lane): waits for a segment's last row, issues its
 //     9 x cin / 16 MMAs into one of two TMEM accumulators, commits them to an
-//     mbarrier, and copies the next row into the slot the previous segment
-//     has finished with;
+//     mbarrier, and copies a row ahead into the slot the previous segment has
+//     finished with;
 //   warps 0-3: read the finished accumulator (warp w owns TMEM lanes
 //     32w..32w+31, one output pixel per lane), release it, add the bias,
 //     apply the ReLU and store FP16.
@@ -49,10 +49,26 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 
 // Shared-memory matrix descriptor (tcgen05): start address, leading (K) and
 // stride (M/N) byte offsets, each >> 4; bits 46-48 = 0b001; base offset 0,
-// relative leading offset, no swizzle.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
+// relative leading offset, no swizzle. The low word holds the address and the
+// leading offset, the high word the stride (128 bytes here) and the constant.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) {
+    return ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16);
+}
+constexpr uint32_t DESC_HI = (128u >> 4) | (1u << 14);
+// D (+)= A B on one 128 x N x 16 step, issued by the warp's elected lane; the
+// first step of a segment overwrites.
+__device__ __forceinline__ void mma(uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, int accumulate,
+                                    uint32_t elected) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}\n" ::"r"(acc),
+        "r"(da), "r"(db), "r"(idesc), "r"(accumulate), "r"(DESC_HI), "r"(elected));
+}
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(one));
+    return one;
 }
 // Instruction descriptor, kind::f16: FP32 accumulator (bits 4-5 = 1), FP16 A
 // and B (bits 7-9, 10-12 = 0), both K-major (bits 15, 16 = 0), N >> 3 at bits
@@ -83,35 +99,50 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 
 constexpr int TC_M = 128;                     // output pixels per segment (TMEM lanes)
 constexpr int HALO = TC_M + 2;                // input pixels per row slice
-constexpr int SLICE = HALO * 16;              // bytes of one 8-channel slice of a row (one TMA box)
-constexpr int SLICE_STRIDE = 136 * 16;        // its stride in shared memory, a multiple of the 128 bytes TMA
-                                              // destinations need: the A operand's LBO
+constexpr int SLICE = HALO * 16;              // bytes of one 8-channel slice of a row: the A operand's LBO
 constexpr int EPI_THREADS = 128;              // warps 0-3
 constexpr int TC_THREADS = EPI_THREADS + 32;  // + warp 4, the issuing warp
+constexpr int RING_MAX = 8;                   // row slots: a segment reads three, the others load ahead
 
 __host__ __device__ constexpr uint32_t tmem_cols(int np) {
     return 2 * np <= 32 ? 32 : 2 * np <= 64 ? 64 : 2 * np <= 128 ? 128 : 2 * np <= 256 ? 256 : 512;
 }
-// Row slots of the ring: four (a segment reads three while the next row
-// loads), or three where that fits twice as many CTAs in an SM's shared memory
-// (the next row then loads once the segment's MMAs are done with its slot).
-constexpr int RING = 4;
-// Weights, the ring of row slots, and slack to align the ring to 1024 bytes.
-static size_t tc_smem(int np, int cin, int ring = RING) {
-    return 9 * (size_t)np * 2 * cin + ring * (size_t)(cin / 8) * SLICE_STRIDE + 1024;
+// A row slot's bytes, a multiple of the 128 a TMA destination needs.
+__host__ __device__ constexpr uint32_t slot_bytes(int cin) { return ((uint32_t)(cin / 8) * SLICE + 127u) & ~127u; }
+// Weights, a segment's output, the ring of row slots, and slack to align to 1024 bytes.
+static size_t tc_smem(int np, int cin, int ring) {
+    return 9 * (size_t)np * 2 * cin + (size_t)TC_M * 2 * np + (size_t)ring * slot_bytes(cin) + 1024;
 }
 
-template <int NP, int RING>
-__global__ void __launch_bounds__(TC_THREADS) k_conv3x3_tc(const __grid_constant__ CUtensorMap rows, int n, int h,
+// What bounded it and no longer does (1024^2, 32 -> 32 channels, 65 -> 46 us;
+// 16 -> 32 56 -> 39; 512^2 112 -> 48 76 -> 52; the same values to the bit):
+// - one row ahead only, so a CTA's period per segment was a row copy's latency
+//   (2 us): the ring holds as many rows as fit (loads_ahead);
+// - one divergent lane's issue, 107 cycles per MMA: the whole warp walks the
+//   segments, so that addresses live in uniform registers (1024^2 80 -> 32
+//   with one CTA per SM 137 -> 86-92 us);
+// - 4-7 us of staging weights by divisions and half sectors before the first
+//   row was asked for: the rows are asked for first, the weights come in whole
+//   sectors;
+// - stores of 16-byte pieces, channels apart: a warp's pixels leave as one
+//   bulk copy.
+// What bounds it now: the MMAs' A operand, 4 KB of shared memory per 128 x N x
+// 16 MMA (32 cycles whatever N is), and at 1024^2 with few channels the
+// epilogue's chain per segment.
+template <int NP>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_conv3x3_tc(const __grid_constant__ CUtensorMap rows, int n, int h,
                                                            int w, int cin, const __half* __restrict__ wt,
                                                            const float* __restrict__ bias, int cout, int relu,
-                                                           __half* __restrict__ y, int run_rows) {
+                                                           __half* __restrict__ y, int run_rows, int ring) {
     constexpr uint32_t COLS = tmem_cols(NP);
     constexpr uint32_t IDESC = instr_desc(TC_M, NP);
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bars[RING + 4];  // full[RING] (TMA), mma[2] (tcgen05.commit), free[2]
+    __shared__ __align__(8) uint64_t bars[RING_MAX + 4];  // full[ring] (TMA), then mma[2] (tcgen05.commit), free[2]
+    __shared__ __align__(16) float bias_s[NP];
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // The warp's number by a shuffle: the compiler then knows it uniform, and
+    // keeps the issuing warp's addresses in uniform registers.
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int chunks = cin >> 3;
     const int per_row = w / TC_M;
     // This CTA's run: column (image, segment) blockIdx.x % columns, rows
@@ -121,35 +152,63 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3x3_tc(const __grid_constant
     const int img = column / per_row, x0 = (column - img * per_row) * TC_M;
     const int y0 = run * run_rows, y1 = min(h, y0 + run_rows);
     const int ntiles = y1 > y0 ? y1 - y0 : 0;
-    const uint32_t wbase = smem_u32(smem);
-    const uint32_t w_tap = NP * 2 * cin;                        // one tap's weights
-    const uint32_t hbase = (wbase + 9 * w_tap + 1023u) & ~1023u;  // the ring of row slots
-    const uint32_t seg = chunks * SLICE_STRIDE;                 // one row slot
-    const uint32_t full0 = smem_u32(&bars[0]), mma0 = smem_u32(&bars[RING]), free0 = smem_u32(&bars[RING + 2]);
+    // Its output channels: all of them, or the group blockIdx.y's.
+    const int co0 = blockIdx.y * NP, cog = min(NP, cout - co0);
+    wt += (long)co0 * 9 * cin;
+    const uint32_t w_tap = NP * 2 * cin;  // one tap's weights
+    const uint32_t seg = slot_bytes(cin);
+    const uint32_t hbase = (smem_u32(smem) + 1023u) & ~1023u;  // the ring of row slots
+    const uint32_t wbase = hbase + ring * seg;
+    const uint32_t obase = wbase + 9 * w_tap;  // a segment's output, 32 pixels per warp
+    const uint32_t full0 = smem_u32(&bars[0]), mma0 = smem_u32(&bars[RING_MAX]), free0 = smem_u32(&bars[RING_MAX + 2]);
 
+    // Relative row q of the run is image row y0 - 1 + q, in slot q % ring; its
+    // copy is that slot's (q / ring)-th: one box of the row's 16-byte channel
+    // slices, each of 130 pixels.
+    const uint32_t bytes = chunks * SLICE;
+    auto load_row = [&](int q, int slot) {
+        const uint32_t bar = full0 + 8 * slot;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+            " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(hbase + slot * seg),
+            "l"((uint64_t)&rows), "r"(0), "r"(x0 - 1), "r"(0), "r"(y0 - 1 + q), "r"(img), "r"(bar)
+            : "memory");
+    };
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"(COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (tid == 0) {
-        for (int k = 0; k < RING; k++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * k));
+    if (tid == EPI_THREADS) {
+        for (int k = 0; k < ring; k++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * k));
         for (int k = 0; k < 2; k++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mma0 + 8 * k));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(free0 + 8 * k), "r"(EPI_THREADS));
         }
-        asm volatile("fence.mbarrier_init.release.cluster;");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (ntiles > 0)
+            for (int q = 0; q < min(ring, ntiles + 2); q++) load_row(q, q);
     }
-    // Every tap's weights, rows padded to NP with zeros: 16-byte copies by all threads.
+    __syncwarp();
+    // Every tap's weights, rows padded to NP with zeros. Sixteen lanes copy
+    // two 16-byte slices of eight rows: whole 32-byte sectors of global memory,
+    // 128 consecutive bytes of shared memory per slice.
     {
-        const int per_tap = NP * chunks;
-        for (int j = tid; j < 9 * per_tap; j += TC_THREADS) {
-            const int tap = j / per_tap, rem = j - tap * per_tap;
-            const int r = rem % NP, c = rem / NP;
-            const bool ok = r < cout;
-            const __half* src = ok ? wt + ((long)r * 9 + tap) * cin + c * 8 : wt;
-            cp_async16(wbase + tap * w_tap + c * (NP * 16) + r * 16, src, ok);
+        const int half = tid >> 4, r8 = tid & 7, c1 = (tid >> 3) & 1;
+        for (int u = half; u < 9 * (NP / 8); u += TC_THREADS / 16) {
+            const int tap = u % 9, r = (u / 9) * 8 + r8;
+            const bool ok = r < cog;
+            const __half* src = ok ? wt + ((long)r * 9 + tap) * cin + c1 * 8 : wt;
+            uint32_t dst = wbase + tap * w_tap + c1 * (NP * 16) + r * 16;
+            for (int c = 0; c < chunks; c += 2) {
+                cp_async16(dst, src, ok);
+                dst += 2 * NP * 16;
+                if (ok) src += 16;
+            }
         }
+        for (int c = tid; c < NP; c += TC_THREADS) bias_s[c] = bias && c < cog ? bias[co0 + c] : 0.0f;
         asm volatile("cp.async.commit_group;");
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
@@ -160,104 +219,134 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3x3_tc(const __grid_constant
     const uint32_t tmem = tmem_slot;
 
     if (warp == 4) {
-        if (lane == 0 && ntiles > 0) {
-            const uint32_t bytes = chunks * SLICE;
-            // Relative row q of the run is image row y0 - 1 + q, in slot q % RING;
-            // its copy is that slot's (q / RING)-th.
-            auto load_row = [&](int q) {
-                const uint32_t bar = full0 + 8 * (q % RING);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-                for (int c = 0; c < chunks; c++) {
-                    const uint32_t dst = hbase + (q % RING) * seg + c * SLICE_STRIDE;
-                    asm volatile(
-                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-                        "l"((uint64_t)&rows), "r"(c * 8), "r"(x0 - 1), "r"(y0 - 1 + q), "r"(img), "r"(bar)
-                        : "memory");
-                }
-            };
-            load_row(0);
-            load_row(1);
-            load_row(2);
+        // The whole warp walks the segments (its addresses stay uniform), the
+        // elected lane issues.
+        const uint32_t elected = elect_one();
+        if (ntiles > 0) {
+            bar_wait(full0, 0);  // rows y-1 and y of the first segment
+            bar_wait(full0 + 8, 0);
+            int first = 0, third = 2, phase = 0;  // slots of rows i and i + 2, the latter's copy
             for (int i = 0; i < ntiles; i++) {
                 const int b = i & 1;
-                for (int q = i; q < i + 3; q++) bar_wait(full0 + 8 * (q % RING), (q / RING) & 1);  // rows y-1, y, y+1
+                bar_wait(full0 + 8 * third, phase);
                 if (i >= 2) bar_wait(free0 + 8 * b, ((i >> 1) - 1) & 1);  // accumulator b read out
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + b * NP;
-                for (int tap = 0; tap < 9; tap++) {
-                    const uint32_t a0 = hbase + ((i + tap / 3) % RING) * seg + (tap % 3) * 16;
-                    const uint32_t b0 = wbase + tap * w_tap;
-                    for (int k = 0; k < cin / 16; k++) {
-                        const uint64_t da = smem_desc(a0 + k * 2 * SLICE_STRIDE, SLICE_STRIDE, 128);
-                        const uint64_t db = smem_desc(b0 + k * 2 * NP * 16, NP * 16, 128);
-                        const uint32_t accumulate = (tap > 0 || k > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(acc),
-                            "l"(da), "l"(db), "r"(IDESC), "r"(accumulate));
+                // The descriptors' low words: the operands' addresses move by
+                // constants, so one thread keeps the tensor pipe fed.
+                const uint32_t tap_step = (cin / 16) * 2 * SLICE / 16;
+                uint32_t db = desc_lo(wbase, NP * 16);
+                int slot = first;
+                for (int dy = 0; dy < 3; dy++) {
+                    uint32_t da = desc_lo(hbase + slot * seg, SLICE);
+                    for (int dx = 0; dx < 3; dx++) {
+#pragma unroll 1
+                        for (int k = 0; k < cin / 16; k++) {
+                            mma(acc, da, db, IDESC, dy + dx + k, elected);
+                            da += 2 * SLICE / 16;
+                            db += 2 * NP;
+                        }
+                        da += 1 - tap_step;  // one pixel on
                     }
+                    slot = slot + 1 == ring ? 0 : slot + 1;
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                if (elected) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                  mma0 + 8 * b)
                              : "memory");
-                if (i + 1 < ntiles) {
-                    // The next segment's new row goes into the slot of row
-                    // i + 3 - RING, which segment i + 3 - RING's MMAs were the
-                    // last to read (the previous segment's with four slots, this
-                    // one's with three).
-                    const int last = i + 3 - RING;
-                    if (last >= 0) bar_wait(mma0 + 8 * (last & 1), (last >> 1) & 1);
-                    load_row(i + 3);
+                // Row i - 1 was last read by the previous segment's MMAs: its
+                // slot takes row i - 1 + ring. Three slots are all this
+                // segment's, whose own MMAs free the first.
+                const int last = i - (ring > 3);
+                if (last >= 0 && last + ring < ntiles + 2) {
+                    bar_wait(mma0 + 8 * (last & 1), (last >> 1) & 1);
+                    if (elected) load_row(last + ring, last == i ? first : first == 0 ? ring - 1 : first - 1);
+                }
+                first = first + 1 == ring ? 0 : first + 1;
+                if (++third == ring) {
+                    third = 0;
+                    phase ^= 1;
                 }
             }
         }
         __syncwarp();
     } else {
-        // Epilogue: warps 0-3, one output pixel per thread.
+        // Epilogue: warps 0-3, one output pixel per thread; a warp's 32 pixels
+        // are consecutive in memory and leave as one bulk copy. With groups of
+        // channels they are not: each pixel's go out by themselves, in whole
+        // sectors.
+        const uint32_t out = obase + warp * 64 * cout;
+        const bool whole = cog == cout;
         for (int i = 0; i < ntiles; i++) {
             const int b = i & 1;
             const bool ok = bar_wait(mma0 + 8 * b, (i >> 1) & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t packed[NP / 2];
+            uint32_t r[NP];
             const uint32_t row_addr = tmem + b * NP + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
             for (int c0 = 0; c0 < NP; c0 += 16) {
-                uint32_t r[16];
+                uint32_t* q = r + c0;
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
                     "[%16];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                      "=r"(r[15])
+                    : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
+                      "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]),
+                      "=r"(q[15])
                     : "r"(row_addr + c0));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    float v0 = __uint_as_float(r[2 * j]), v1 = __uint_as_float(r[2 * j + 1]);
-                    const int co = c0 + 2 * j;
-                    if (bias && co < cout) v0 += __ldg(bias + co);
-                    if (bias && co + 1 < cout) v1 += __ldg(bias + co + 1);
-                    if (relu) {
-                        v0 = fmaxf(v0, 0.0f);
-                        v1 = fmaxf(v1, 0.0f);
-                    }
-                    packed[c0 / 2 + j] = (uint32_t)__half_as_ushort(__float2half_rn(v0)) |
-                                         ((uint32_t)__half_as_ushort(__float2half_rn(v1)) << 16);
-                }
             }
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            // The values are used only after the wait.
+#pragma unroll
+            for (int c = 0; c < NP; c++) asm volatile("" : "+r"(r[c]));
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(free0 + 8 * b) : "memory");
-            if (ok) {
-                const long p = ((long)img * h + y0 + i) * w + x0 + tid;
-                __half* dst = y + p * cout;
+            // The warp's previous copy has read its pixels.
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
 #pragma unroll
-                for (int c0 = 0; c0 < NP; c0 += 8)
-                    if (c0 < cout)
-                        *(uint4*)(dst + c0) = make_uint4(packed[c0 / 2], packed[c0 / 2 + 1], packed[c0 / 2 + 2],
-                                                         packed[c0 / 2 + 3]);
+            for (int c0 = 0; c0 < NP; c0 += 8) {
+                if (c0 >= cog) continue;
+                uint32_t packed[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                    const float4 add = *(const float4*)(bias_s + c0 + j);
+                    float v[4] = {__uint_as_float(r[c0 + j]), __uint_as_float(r[c0 + j + 1]),
+                                  __uint_as_float(r[c0 + j + 2]), __uint_as_float(r[c0 + j + 3])};
+                    if (bias) {
+                        v[0] += add.x;
+                        v[1] += add.y;
+                        v[2] += add.z;
+                        v[3] += add.w;
+                    }
+                    if (relu)
+                        for (int k = 0; k < 4; k++) v[k] = fmaxf(v[k], 0.0f);
+                    for (int k = 0; k < 2; k++)
+                        packed[j / 2 + k] = (uint32_t)__half_as_ushort(__float2half_rn(v[2 * k])) |
+                                            ((uint32_t)__half_as_ushort(__float2half_rn(v[2 * k + 1])) << 16);
+                }
+                if (!whole) {
+                    if (ok)
+                        *(uint4*)(y + (((long)img * h + y0 + i) * w + x0 + tid) * cout + co0 + c0) =
+                            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    continue;
+                }
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out + (lane * cout + c0) * 2),
+                             "r"(packed[0]), "r"(packed[1]), "r"(packed[2]), "r"(packed[3])
+                             : "memory");
+            }
+            if (!whole) continue;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0 && ok) {
+                const long p = ((long)img * h + y0 + i) * w + x0 + warp * 32;
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                                 (uint64_t)__cvta_generic_to_global(y + p * cout)),
+                             "r"(out), "r"(64 * cout)
+                             : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        __syncwarp();
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -265,8 +354,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3x3_tc(const __grid_constant
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
 }
 
-// The input tensor (n, h, w, cin) FP16 as a 4-D TMA map, innermost first:
-// channels, pixels, rows, images; boxes of 8 channels x 130 pixels x 1 x 1.
+// The input tensor (n, h, w, cin) FP16 as a 5-D TMA map, innermost first: the
+// channels of a slice, pixels, slices, rows, images; a box is one row's slices
+// of 130 pixels.
 static bool encode_rows_map(CUtensorMap* map, const void* x, int n, int h, int w, int cin) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
@@ -277,14 +367,17 @@ static bool encode_rows_map(CUtensorMap* map, const void* x, int n, int h, int w
             return false;
         encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
-    const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    const cuuint64_t strides[3] = {(cuuint64_t)cin * 2, (cuuint64_t)w * cin * 2, (cuuint64_t)h * w * cin * 2};
-    const cuuint32_t box[4] = {8, HALO, 1, 1};
-    const cuuint32_t elem[4] = {1, 1, 1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(x), dims, strides, box, elem,
+    const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)(cin / 8), (cuuint64_t)h, (cuuint64_t)n};
+    const cuuint64_t strides[4] = {(cuuint64_t)cin * 2, 16, (cuuint64_t)w * cin * 2, (cuuint64_t)h * w * cin * 2};
+    const cuuint32_t box[5] = {8, HALO, (cuuint32_t)(cin / 8), 1, 1};
+    const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(x), dims, strides, box, elem,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+// The shared memory a block may ask for, beside its static variables.
+constexpr int TC_SMEM_MAX = 226 * 1024;
 
 // Resident CTAs per SM for `smem` bytes of dynamic shared memory: by shared
 // memory (with 1 KB per CTA the system reserves and the static barriers), by
@@ -297,65 +390,83 @@ static int resident_ctas(size_t smem, int np, int sm_smem) {
     return per_sm < 1 ? 1 : per_sm;
 }
 
-template <int NP, int RING>
-static cudaError_t launch_tc(const CUtensorMap& map, int n, int h, int w, int cin, const __half* wt, const float* bias,
-                             int cout, int relu, __half* y, cudaStream_t s, int sms, int per_sm) {
-    const size_t smem = tc_smem(NP, cin, RING);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e =
-            cudaFuncSetAttribute(k_conv3x3_tc<NP, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
-    // Runs of rows: every resident CTA takes one, the runs of a column of
-    // segments as long as the CTAs per column allow.
-    const long columns = (long)n * (w / TC_M);
-    const long slots = (long)sms * per_sm;
-    const long per_column = std::max(1L, slots / columns);
-    const int run_rows = (int)((h + per_column - 1) / per_column);
-    const long grid = columns * ((h + run_rows - 1) / run_rows);
-    k_conv3x3_tc<NP, RING><<<(unsigned)grid, TC_THREADS, smem, s>>>(map, n, h, w, cin, wt, bias, cout, relu, y,
-                                                                    run_rows);
-    return cudaGetLastError();
+// CTAs per SM, at most four, then the row slots that leave room for them.
+// 1024^2, 16 -> 32 / 32 -> 32 / 32 -> 8 channels: one CTA per SM 61.7 / 65.8 /
+// 59.7 us, four 39.2 / 47.5 / 35.0. An earlier form of the kernel: six CTAs
+// against four 43.5 and 39.5 us (16 -> 32), four, six and eight slots 59.7,
+// 51.4 and 51.4 us (32 -> 32).
+static void loads_ahead(int np, int cin, int sm_smem, int fewest, int* ring, int* per_sm) {
+    *per_sm = std::min(4, resident_ctas(tc_smem(np, cin, fewest), np, sm_smem));
+    *ring = fewest;
+    while (*ring < RING_MAX && tc_smem(np, cin, *ring + 1) <= TC_SMEM_MAX &&
+           resident_ctas(tc_smem(np, cin, *ring + 1), np, sm_smem) >= *per_sm)
+        ++*ring;
 }
 
-// Four row slots, or three where that fits more CTAs per SM (the U-Net's
-// full-resolution decoder, 80 -> 32 channels: one CTA per SM with four slots,
-// two with three).
 template <int NP>
-static cudaError_t launch_tc_ring(const CUtensorMap& map, int n, int h, int w, int cin, const __half* wt,
-                                  const float* bias, int cout, int relu, __half* y, cudaStream_t s) {
+static cudaError_t launch_tc(const CUtensorMap& map, int n, int h, int w, int cin, const __half* wt, const float* bias,
+                             int cout, int relu, __half* y, cudaStream_t s, int groups, int fewest) {
     int dev = 0, sms = 0, sm_smem = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
     if (e != cudaSuccess) return e;
-    const int four = resident_ctas(tc_smem(NP, cin, 4), NP, sm_smem);
-    const int three = resident_ctas(tc_smem(NP, cin, 3), NP, sm_smem);
-    if (four == 1 && three > 1)
-        return launch_tc<NP, 3>(map, n, h, w, cin, wt, bias, cout, relu, y, s, sms, three);
-    return launch_tc<NP, 4>(map, n, h, w, cin, wt, bias, cout, relu, y, s, sms, four);
+    static bool configured = false;
+    if (!configured) {
+        e = cudaFuncSetAttribute(k_conv3x3_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX);
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    int ring = 0, per_sm = 0;
+    loads_ahead(NP, cin, sm_smem, fewest, &ring, &per_sm);
+    const size_t smem = tc_smem(NP, cin, ring);
+    // Runs of rows: every resident CTA takes one, the runs of a column of
+    // segments as long as the CTAs per column allow.
+    const long columns = (long)n * (w / TC_M);
+    const long slots = (long)sms * per_sm;
+    const long per_column = std::max(1L, slots / (columns * groups));
+    const int run_rows = (int)((h + per_column - 1) / per_column);
+    const long grid = columns * ((h + run_rows - 1) / run_rows);
+    k_conv3x3_tc<NP><<<dim3((unsigned)grid, groups), TC_THREADS, smem, s>>>(map, n, h, w, cin, wt, bias, cout, relu, y, run_rows,
+                                                              ring);
+    return cudaGetLastError();
 }
 
 // The tensor-core convolution when the shape suits it (widths that are
-// multiples of 128, cout <= 96 and the weights and two segments' rows within
-// 220 KB of shared memory); returns false to leave the shape to the mma.sync
-// convolution. *err receives the launch's error.
+// multiples of 128, and the weights, a segment's output and the rows within
+// 226 KB of shared memory); returns false to leave the shape to the mma.sync
+// convolution. Up to 96 output channels whose weights fit beside four rows run
+// as one group. With `grouped`, the others are split into the fewest groups
+// that fit beside four rows, or three (each group reads the input again):
+// against mma.sync 256^2 144 -> 64 channels 83 -> 39 us (two groups), 128^2
+// 176 -> 80 41 -> 31 (five), four images of 256^2 64 -> 144 230 -> 78 (two),
+// of 128^2 80 -> 176 94 -> 35 (two), one of 8 x 128 144 -> 64 18.7 -> 13.0.
+// *err receives the launch's error.
 bool conv3x3_tc(const __half* x, int n, int h, int w, int cin, const __half* wt, const float* bias, int cout,
-                int relu, __half* y, cudaStream_t s, cudaError_t* err) {
-    const int np = (cout + 15) / 16 * 16;
-    if (w % TC_M || np > 96 || tc_smem(np, cin) > 220 * 1024) return false;
+                int relu, __half* y, cudaStream_t s, bool grouped, cudaError_t* err) {
+    if (w % TC_M) return false;
     if (((uintptr_t)x | (uintptr_t)wt | (uintptr_t)y) % 16) return false;
+    int np = (cout + 15) / 16 * 16, groups = 1, fewest = 4;
+    if (np > 96 || tc_smem(np, cin, 4) > TC_SMEM_MAX) {
+        if (!grouped) return false;
+        const int wide = np;
+        for (groups = 2;; groups++) {
+            np = ((wide + groups - 1) / groups + 15) / 16 * 16;
+            fewest = tc_smem(np, cin, 4) <= TC_SMEM_MAX ? 4 : 3;
+            if (np <= 96 && tc_smem(np, cin, fewest) <= TC_SMEM_MAX) break;
+            if (np == 16) return false;
+        }
+        groups = (wide + np - 1) / np;
+    }
     CUtensorMap map;
     if (!encode_rows_map(&map, x, n, h, w, cin)) return false;
     switch (np) {
-        case 16: *err = launch_tc_ring<16>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
-        case 32: *err = launch_tc_ring<32>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
-        case 48: *err = launch_tc_ring<48>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
-        case 64: *err = launch_tc_ring<64>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
-        case 80: *err = launch_tc_ring<80>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
-        case 96: *err = launch_tc_ring<96>(map, n, h, w, cin, wt, bias, cout, relu, y, s); break;
+        case 16: *err = launch_tc<16>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
+        case 32: *err = launch_tc<32>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
+        case 48: *err = launch_tc<48>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
+        case 64: *err = launch_tc<64>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
+        case 80: *err = launch_tc<80>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
+        case 96: *err = launch_tc<96>(map, n, h, w, cin, wt, bias, cout, relu, y, s, groups, fewest); break;
         default: return false;
     }
     return true;
@@ -373,7 +484,7 @@ extern "C" vv_status vv_nn_conv3x3_tc(const void* x, int n, int h, int w, int ci
         return VV_ERR_ARG;
     cudaError_t e = cudaSuccess;
     if (!conv3x3_tc((const __half*)x, n, h, w, cin, (const __half*)weights, bias, cout, relu, (__half*)y,
-                    (cudaStream_t)stream, &e))
+                    (cudaStream_t)stream, false, &e))
         return VV_ERR_ARG;
     return e == cudaSuccess ? VV_OK : VV_ERR_CUDA;
 }

@@ -288,6 +288,20 @@ def test_tensor_core_convolution_long_runs(lib, cin, cout):
     assert lib.vv_nn_tc_status(C.byref(failed), 1) == 0 and failed.value == 0
 
 
+# One-pixel rows, a row longer than a block's four pixels per thread, more than
+# 256 pieces per pixel.
+@pytest.mark.parametrize("shape", [(1, 3, 1, 8, 8), (3, 2, 7, 24, 16), (1, 2, 300, 96, 80), (2, 3, 2, 1032, 1040)])
+def test_upsample_concat_shapes(lib, shape):
+    n, h, w, ca, cb = shape
+    torch.manual_seed(sum(shape))
+    a = torch.randn((n, h, w, ca), device="cuda").half()
+    b = torch.randn((n, 2 * h, 2 * w, cb), device="cuda").half()
+    y = torch.zeros((n, 2 * h, 2 * w, ca + cb), dtype=torch.float16, device="cuda")
+    assert lib.vv_nn_upsample_concat(a.data_ptr(), n, h, w, ca, b.data_ptr(), cb, y.data_ptr(), S) == 0
+    up = a.repeat_interleave(2, 1).repeat_interleave(2, 2)
+    assert torch.equal(y, torch.cat([up, b], 3))
+
+
 # Output channels in groups: 2 of 32 beside three rows, 5 of 16 beside three, 2 of 64
 # (the last of 48), 2 of 80 (the last of 64), 2 of 96 (the last of 80); one-row images.
 @pytest.mark.parametrize("shape", [(1, 5, 256, 144, 64), (1, 9, 128, 176, 80), (2, 3, 128, 48, 112),

@@ -142,17 +142,21 @@ __device__ __forceinline__ float ign(float px, float py) {
     return b - floorf(b);
 }
 
-// A lighting volume, sampled as the border sampler does: linear between texel
-// centres, texels outside the volume white (1, 1, 1, 1).
+// The shadow volume while slice `slice` of `axis` is written, sampled as the border
+// sampler does: linear between texel centres, texels outside the volume white
+// (1, 1, 1, 1). A lookup at the slice before lands within rounding of that slice's
+// texels, so it may also weigh the slice being written, by up to 1e-5: those texels
+// count as 0, as they are before the launch, and not as whatever other threads
+// have written by then.
 struct LightVol {
-    const uint16_t* data;  // `channels` halves per texel, x fastest
-    int w, h, d, channels;
+    const ushort4* data;  // RGBA16F, x fastest
+    int w, h, d, axis, slice;
 };
 __device__ __forceinline__ float4 lv_texel(const LightVol& v, int x, int y, int z) {
     if (x < 0 || y < 0 || z < 0 || x >= v.w || y >= v.h || z >= v.d) return make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if ((v.axis == 0 ? x : v.axis == 1 ? y : z) == v.slice) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     long i = ((long)z * v.h + y) * v.w + x;
-    if (v.channels == 1) return make_float4(h2f(__ldg(v.data + i)), 0.0f, 0.0f, 1.0f);
-    ushort4 t = __ldg((const ushort4*)v.data + i);
+    ushort4 t = __ldg(v.data + i);
     return make_float4(h2f(t.x), h2f(t.y), h2f(t.z), h2f(t.w));
 }
 __device__ float4 lv_linear(const LightVol& v, f3 tc) {
@@ -371,7 +375,7 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     const float4 f = GIVEN ? __ldg(factors + at) : shadow_factors(A, w, here);
     if (GIVEN) asm volatile("griddepcontrol.wait;" ::: "memory");
     f3 prev = here + w.l_idx * w.s;
-    LightVol V{(const uint16_t*)vol, sx, sy, sz, 4};
+    LightVol V{vol, sx, sy, sz, axis, slice};
     float4 back = lv_linear(V, (prev + 0.5f) / w.dims);
     float direct = back.w * f.w;
     f3 axis_u = mk(0.0f), axis_v = mk(0.0f);

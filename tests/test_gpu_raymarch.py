@@ -109,3 +109,45 @@ def test_lanes_per_ray_give_the_same_image(small_cfg, gpu_ctx, monkeypatch, size
             assert np.array_equal(hdr, images[0][0]) and np.array_equal(out, images[0][1])
     finally:
         r.destroy()
+
+
+AXES = {"+x": (90.0, 0.0), "-x": (-90.0, 0.0), "+y": (180.0, 0.0), "-y": (0.0, 0.0), "+z": (0.0, 90.0),
+        "-z": (0.0, -90.0)}  # the key light's azimuth and elevation as seen by a camera that looks along +y
+
+
+@pytest.mark.parametrize("tilt", [0.0, 11.0])
+@pytest.mark.parametrize("towards", AXES)
+def test_shadow_sweep_with_and_without_room_for_its_factors(gpu_ctx, towards, tilt):
+    """The sweep whose factors are taken ahead, slices chained (a renderer with
+    label masks has the room), against the sweep of plain launches (one without
+    has none): the same volume bit by bit, along each axis both ways. Both
+    renderers draw the transfer function alone."""
+    rng = np.random.default_rng(5)
+    dims = (75, 58, 66)  # 38 x 29 x 33 texels, blocks of 8 x 8 partly outside
+    hu = rng.integers(-1000, 1500, dims[::-1]).astype(np.int16)
+    cfg = dict(min_spacing=1.0, label_params=abi.label_params_default())
+    volume = abi.volume_struct(hu, (1.0, 1.0, 1.0))
+    sweeps = []
+    for labels in (None, np.zeros(hu.shape, np.uint8)):
+        r = R.Renderer(gpu_ctx, volume, abi.tf_struct(abi.PRESETS["bone"]))
+        try:
+            if labels is not None:
+                r.set_labels(labels)
+            p = scene.frame_params_for(cfg, list(r.center), r.diagonal)
+            p.path_tracing.enabled = 0
+            p.camera.pitch = p.camera.yaw = 0.0
+            azimuth, elevation = AXES[towards]
+            p.lighting.azimuth = abi.to_radians(azimuth + tilt)
+            p.lighting.elevation = abi.to_radians(elevation + (tilt if abs(elevation) < 90.0 else -tilt))
+            r.resize(16, 16)
+            for _ in range(2):  # twice: with the light moved between, so that both are swept
+                p.lighting.elevation, other = abi.f32(0.3), p.lighting.elevation
+                r.record(1, p)
+                p.lighting.elevation = other
+                r.record(2, p)
+                sweeps.append(r.read_volume(abi.VOLUME_SHADOW))
+        finally:
+            r.destroy()
+    assert _half(sweeps[0]).std() > 0.05
+    for s in sweeps[1:]:
+        assert np.array_equal(s, sweeps[0])

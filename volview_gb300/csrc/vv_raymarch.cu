@@ -148,18 +148,23 @@ __device__ __forceinline__ float ign(float px, float py) {
 // texels, so it may also weigh the slice being written, by up to 1e-5: those texels
 // count as 0, as they are before the launch, and not as whatever other threads
 // have written by then.
+// CHAINED: the launch that writes the texels read here may still have been
+// running when the reading one started, so the read-only path, which is for data
+// that does not change while a kernel lives, is not for them. The loads are
+// coherent ones from L2, since L1 may hold a sector from before (with x as the
+// sweep's axis one sector holds texels of several slices).
 struct LightVol {
     const ushort4* data;  // RGBA16F, x fastest
     int w, h, d, axis, slice;
 };
-__device__ __forceinline__ float4 lv_texel(const LightVol& v, int x, int y, int z) {
+template <bool CHAINED> __device__ __forceinline__ float4 lv_texel(const LightVol& v, int x, int y, int z) {
     if (x < 0 || y < 0 || z < 0 || x >= v.w || y >= v.h || z >= v.d) return make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     if ((v.axis == 0 ? x : v.axis == 1 ? y : z) == v.slice) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     long i = ((long)z * v.h + y) * v.w + x;
-    ushort4 t = __ldg(v.data + i);
+    ushort4 t = CHAINED ? __ldcg(v.data + i) : __ldg(v.data + i);
     return make_float4(h2f(t.x), h2f(t.y), h2f(t.z), h2f(t.w));
 }
-__device__ float4 lv_linear(const LightVol& v, f3 tc) {
+template <bool CHAINED> __device__ float4 lv_linear(const LightVol& v, f3 tc) {
     float x = tc.x * (float)v.w - 0.5f, y = tc.y * (float)v.h - 0.5f, z = tc.z * (float)v.d - 0.5f;
     int i0 = (int)floorf(x), j0 = (int)floorf(y), k0 = (int)floorf(z);
     float a = x - (float)i0, b = y - (float)j0, c = z - (float)k0;
@@ -168,7 +173,7 @@ __device__ float4 lv_linear(const LightVol& v, f3 tc) {
         for (int dj = 0; dj < 2; dj++)
             for (int di = 0; di < 2; di++) {
                 float w = (di ? a : 1.0f - a) * (dj ? b : 1.0f - b) * (dk ? c : 1.0f - c);
-                float4 t = lv_texel(v, i0 + di, j0 + dj, k0 + dk);
+                float4 t = lv_texel<CHAINED>(v, i0 + di, j0 + dj, k0 + dk);
                 r.x += t.x * w;
                 r.y += t.y * w;
                 r.z += t.z * w;
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     if (GIVEN) asm volatile("griddepcontrol.wait;" ::: "memory");
     f3 prev = here + w.l_idx * w.s;
     LightVol V{vol, sx, sy, sz, axis, slice};
-    float4 back = lv_linear(V, (prev + 0.5f) / w.dims);
+    float4 back = lv_linear<GIVEN>(V, (prev + 0.5f) / w.dims);
     float direct = back.w * f.w;
     f3 axis_u = mk(0.0f), axis_v = mk(0.0f);
     set3(axis_u, u_axis, A.u.subsurface[2]);
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     for (int i = 0; i < 4; i++) {
         f3 offset = (i & 1) == 0 ? axis_u : axis_v;
         offset *= i < 2 ? 1.0f : -1.0f;
-        float4 t = lv_linear(V, (prev + offset + 0.5f) / w.dims);
+        float4 t = lv_linear<GIVEN>(V, (prev + offset + 0.5f) / w.dims);
         gathered += 0.15f * mk(t.x, t.y, t.z);
     }
     f3 indirect = gathered * mk(f.x, f.y, f.z);

@@ -151,3 +151,35 @@ def test_shadow_sweep_with_and_without_room_for_its_factors(gpu_ctx, towards, ti
     assert _half(sweeps[0]).std() > 0.05
     for s in sweeps[1:]:
         assert np.array_equal(s, sweeps[0])
+
+
+@pytest.mark.parametrize("size", [(16, 16), (37, 21), (96, 64)])
+@pytest.mark.parametrize("mode", [abi.LABEL_HYBRID, abi.LABEL_ISOLATE])
+def test_lanes_per_ray_with_labels_up_to_the_volumes_faces(small_cfg, gpu_ctx, monkeypatch, size, mode):
+    """Labels that fill the volume to its faces, its silhouette inside the image:
+    rays that miss the volume gather nothing, whatever the rays beside them in
+    the warp do, with two and four lanes per ray as with one."""
+    z, y, x = np.mgrid[0:21, 0:27, 0:30]
+    labels = (1 + (x // 5 + y // 4 + z // 6) % 10).astype(np.uint8)
+    hu = (200 + 37 * labels.astype(np.int16)).astype(np.int16)
+    params = abi.LabelParams.from_buffer_copy(bytes(small_cfg["label_params"]))
+    params.mode = mode
+    r = R.Renderer(gpu_ctx, abi.volume_struct(hu, (1.0, 1.0, 1.0)), small_cfg["tf"])
+    try:
+        r.set_labels(labels)
+        p = scene.frame_params_for(dict(min_spacing=1.0, label_params=params), list(r.center), r.diagonal)
+        p.camera.yaw, p.camera.pitch = abi.f32(0.5), abi.f32(0.3)
+        p.path_tracing.enabled = 0
+        r.resize(*size)
+        images = []
+        for lanes in ("1", "2", "4"):
+            monkeypatch.setenv("VV_DVR_LANES", lanes)
+            r.reset_view()
+            r.record(1, p)
+            images.append(r.read_hdr())
+        clear = _half(images[0])[..., 3] == 1.0  # transmittance: nothing met
+        assert 0.1 < clear.mean() < 0.95
+        for image in images[1:]:
+            assert np.array_equal(image, images[0])
+    finally:
+        r.destroy()

@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS)
     f3 v = -dir;
     // The ray's: the same in its lanes.
     f3 radiance = mk(0.0f);
-    float transmittance = 1.0f, pos = 0.0f;
+    float transmittance = 1.0f, pos = INFINITY;  // past its end: a ray that misses the volume never marches
     bool refined = false, marching = inside && t.x < t.y;
     // The lane's sample.
     bool lit = false, has_grad = false;

@@ -16,6 +16,7 @@ import os
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from volview_gb300 import abi, scene
 from volview_gb300 import renderer as R
 
@@ -181,5 +182,50 @@ def test_lanes_per_ray_with_labels_up_to_the_volumes_faces(small_cfg, gpu_ctx, m
         assert 0.1 < clear.mean() < 0.95
         for image in images[1:]:
             assert np.array_equal(image, images[0])
+    finally:
+        r.destroy()
+
+
+@pytest.mark.parametrize("skip", [1, 0])
+@pytest.mark.parametrize("mode", ["plain", "off", "tint"])
+@pytest.mark.parametrize("hu,fmt", [(0, abi.DENSITY_FP16), (0, abi.DENSITY_BF16), (2048, abi.DENSITY_FP16),
+                                    (2048, abi.DENSITY_UNORM16)])
+def test_occlusion_and_shadow_next_to_an_opacity_edge(gpu_ctx, hu, fmt, mode, skip):
+    """A homogeneous volume whose transfer function is opaque up to one HU below
+    it: the lookup between the two LUT entries gives an extinction, although the
+    bucket maximum of the density, which starts one entry higher, is 0. The
+    extinction is constant (the sampler clamps to the volume), so the occlusion
+    is min(2 exp(-15 c), 1) everywhere (16 directions of 8 samples, 15 mm) and
+    each slice of the sweep lets exp(-2 c) through (half resolution, 1 mm).
+    Bars: the occlusion's FP16 ulp and the 8 FP32 adds, 1e-3; a slice's FP16
+    rounding, 2^-11 relative, over 12 slices, 1e-2."""
+    volume = np.full((24, 24, 24), hu, np.int16)
+    tf = abi.tf_struct([(-1024.0, (0.8, 0.7, 0.6), 6.0), (hu - 1.0, (0.8, 0.7, 0.6), 6.0),
+                        (float(hu), (0.8, 0.7, 0.6), 0.0), (3071.0, (0.8, 0.7, 0.6), 0.0)])
+    lp = abi.label_params_default()
+    lp.mode = abi.LABEL_TINT if mode == "tint" else abi.LABEL_OFF
+    struct = abi.volume_struct(volume, (1.0, 1.0, 1.0))
+    cpu = O.CpuRenderer(struct, tf, volume, density_format=fmt)
+    r = R.Renderer(gpu_ctx, struct, tf, abi.precision(density_format=fmt))
+    try:
+        if mode != "plain":
+            r.set_labels(np.zeros(volume.shape, np.uint8))
+        p = scene.frame_params_for(dict(min_spacing=1.0, label_params=lp), list(r.center), r.diagonal)
+        p.path_tracing.enabled = 0
+        p.skip_empty_space = skip
+        p.camera.yaw = p.camera.pitch = 0.0
+        p.lighting.azimuth, p.lighting.elevation = 0.0, abi.to_radians(90.0)  # towards +z
+        r.resize(16, 16)
+        r.record(1, p)
+        c = float(r.probe_extinction(p, [[11.3, 12.1, 10.6]], smooth=False)[0, 2])  # blue: no chroma
+        lp.mode = abi.LABEL_OFF
+        cpu.resize(16, 16)
+        q = scene.frame_params_for(dict(min_spacing=1.0, label_params=lp), list(r.center), r.diagonal)
+        expected, bound = cpu.extinction(q, [[11.3, 12.1, 10.6]], smooth=False)[0, [2, 3]]
+        assert c > 0.02 and abs(c - expected) <= 0.05 * expected and bound == 0.0
+        ao, shadow = _half(r.read_volume(abi.VOLUME_AO)), _half(r.read_volume(abi.VOLUME_SHADOW))
+        assert np.all(np.abs(ao - min(2.0 * np.exp(-15.0 * c), 1.0)) <= 1e-3)
+        through = np.exp(-2.0 * c * np.arange(12, 0, -1))[:, None, None]  # z fastest from the light: the last slice first
+        assert np.all(np.abs(shadow[..., 3] - through) <= 1e-2 * through + 1e-4)
     finally:
         r.destroy()

@@ -34,11 +34,15 @@ __device__ __forceinline__ f3 tex_to_index(const PtArgs& A, f3 tex) { return tex
 
 // common.glsl:385-391: a shadow-ray sample (ghosts and clipped parts cast no
 // shadow; a clipped point's other fields are not read).
-// In a brick whose majorant is 0 (the brick and two voxels around hold no label
-// mask and no opacity) the extinction is 0 without a look at the volume.
+// In the modes that draw labels alone, a brick of majorant 0 holds no label mask,
+// and neither do two voxels around it: the extinction is 0 without a look at the
+// volume. Where the transfer function draws, a majorant of 0 does not say so: a
+// density's bucket maximum starts one LUT entry above the lower of the two entries
+// that the density is interpolated between.
 __device__ Sample sample_point(const PtArgs& A, f3 idx) {
     int plane;
-    if (__ldg(A.majorant + brick_index(A, idx)) <= 0.0f || clip_depth(A, idx, plane) > 0.0f) {
+    const bool skips = A.u.path[3] != 0u && A.u.labels[0] >= 2.0f;
+    if ((skips && __ldg(A.majorant + brick_index(A, idx)) <= 0.0f) || clip_depth(A, idx, plane) > 0.0f) {
         Sample s;
         s.albedo = mk(0.0f);
         s.extinction = 0.0f;

@@ -229,3 +229,29 @@ def test_occlusion_and_shadow_next_to_an_opacity_edge(gpu_ctx, hu, fmt, mode, sk
         assert np.all(np.abs(shadow[..., 3] - through) <= 1e-2 * through + 1e-4)
     finally:
         r.destroy()
+
+
+@pytest.mark.parametrize("preintegrate", [0, 1])
+@pytest.mark.parametrize("size", [(1, 1), (37, 21), (96, 64)])
+def test_transfer_function_alone_as_with_labels_that_draw_nothing(small_cfg, gpu_ctx, size, preintegrate):
+    """Rays wait for more company with labels than without; which rays are lit
+    together changes none of them. Tint over a label volume of zeros draws what
+    the transfer function alone does, bit by bit."""
+    cfg = small_cfg
+    r = R.Renderer(gpu_ctx, cfg["volume"], cfg["tf"])
+    try:
+        r.set_labels(np.zeros(cfg["labels_vol"].shape, np.uint8))
+        p = scene.frame_params_for(cfg, list(r.center), r.diagonal, clip_sagittal=True)
+        p.camera.distance = abi.f32(p.camera.distance * 0.45)
+        p.path_tracing.enabled = 0
+        p.preintegrate = preintegrate
+        r.resize(*size)
+        images = []
+        for mode in (abi.LABEL_OFF, abi.LABEL_TINT):
+            p.labels.mode = mode
+            r.record(1, p)
+            images.append(r.read_hdr())
+        assert size == (1, 1) or np.any(images[0][..., :3])
+        assert np.array_equal(images[0], images[1])
+    finally:
+        r.destroy()

@@ -405,12 +405,14 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
 // by instruction issue: a lit sample costs thousands of instructions (the
 // surface's relief and texture noises, six mask fetches, three lighting
 // lookups), the steps between them a few hundred. A warp (8 x 4 pixels) marches
-// until VV_DVR_GATHER of its rays stand at a sample to light, or none marches,
-// and lights those together. Measured on 512 x 512 x 400 at 1024^2: 28.6 ms per
+// until `gather` of its rays stand at a sample to light, or none marches, and
+// lights those together. Measured on 512 x 512 x 400 at 1024^2: 28.6 ms per
 // frame with the lighting inside each step and 16 noises per relief, 17.4 with
 // the phases and masks read first, 14.4 with the shared noises (relief_heights).
 // Gathering 1, 8, 16, 24, 28, 32 rays: 19.0, 18.6, 18.2, 17.3, 17.0, 17.8 ms
 // there and 21.0, 20.9, 20.6, 21.9, 22.9, 22.4 for a 511 x 387 clip drag.
+// Without labels a lit sample has no relief and no texture and costs little more
+// than a step, so rays that wait for company only lose time: dvr_gather.
 #ifndef VV_DVR_MIN_BLOCKS
 #define VV_DVR_MIN_BLOCKS 4
 #endif
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
 #define VV_DVR_GATHER 24
 #endif
 __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_constant__ PtArgs A, const LightTex SV,
-                                                               const LightTex AV) {
+                                                               const LightTex AV, int gather) {
     int px = blockIdx.x * 8 + (threadIdx.x & 7), py = blockIdx.y * 8 + (threadIdx.x >> 3);
     const bool inside = px < (int)A.u.flags[2] && py < (int)A.u.flags[3];
     float nx = ((float)px + 0.5f) / (float)A.u.flags[2] * 2.0f - 1.0f;
@@ -460,7 +462,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_cons
         for (;;) {
             const unsigned marching = __ballot_sync(0xffffffffu, state == MARCH);
             shading = __ballot_sync(0xffffffffu, state == SHADE);
-            if (!marching || __popc(shading) >= VV_DVR_GATHER) break;
+            if (!marching || __popc(shading) >= gather) break;
             if (state != MARCH) continue;
             if (!(tt < t.y && transmittance > 0.01f)) {
                 state = OUT;
@@ -729,6 +731,12 @@ cudaError_t launch_pad_lighting(const uint16_t* vol, int channels, int w, int h,
     return cudaGetLastError();
 }
 
+// Rays that k_dvr gathers before it lights them. 512^2, a head of 256 x 256 x 200, the
+// transfer function alone: 1, 4, 8, 16, 24 rays 2.6, 2.2, 2.7, 3.0, 3.7 ms, pre-integrated
+// 2.8, 2.8, 3.1, 4.2, 5.0; lighting inside each step 2.7 and 2.9. With labels (Tint)
+// 7.4, 7.6, 6.3, 6.5, 6.8 ms, and pre-integrated Hybrid 8.0 to 8.2 for all.
+static int dvr_gather(const PtArgs& a) { return a.u.labels[0] >= 1.0f ? VV_DVR_GATHER : 4; }
+
 cudaError_t launch_dvr(const PtArgs& a, const LightTex& shadow, const LightTex& ao, cudaStream_t s) {
     // Lanes per ray: four below 3 * 2^17 pixels, where the slowest rays set the
     // time, two above, where lanes past a ray's end cost more than they save, and
@@ -747,7 +755,7 @@ cudaError_t launch_dvr(const PtArgs& a, const LightTex& shadow, const LightTex& 
     else if (lanes == 2)
         k_dvr_masks<2><<<dim3((a.width + 1) / 2, (a.height + 15) / 16), 64, 0, s>>>(a, shadow, ao);
     else
-        k_dvr<<<dim3((a.width + 7) / 8, (a.height + 7) / 8), 64, 0, s>>>(a, shadow, ao);
+        k_dvr<<<dim3((a.width + 7) / 8, (a.height + 7) / 8), 64, 0, s>>>(a, shadow, ao, dvr_gather(a));
     return cudaGetLastError();
 }
 

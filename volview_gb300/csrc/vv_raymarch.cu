@@ -419,6 +419,11 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
 #ifndef VV_DVR_GATHER
 #define VV_DVR_GATHER 24
 #endif
+// MASKS_FIRST: for the modes that draw labels alone, without pre-integration. A
+// drawn label replaces what the transfer function gives there, so a sample outside
+// the masks needs no density (labelled_at); pre-integrated segments take every
+// step's. Launched as the one-lane form of k_dvr_masks only (VV_DVR_LANES=1).
+template <bool MASKS_FIRST>
 __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_constant__ PtArgs A, const LightTex SV,
                                                                const LightTex AV, int gather) {
     int px = blockIdx.x * 8 + (threadIdx.x & 7), py = blockIdx.y * 8 + (threadIdx.x >> 3);
@@ -437,10 +442,6 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_cons
     float step_mm = A.u.dims[3];
     bool preintegrate = A.u.lighting[2] != 0u;
     const uint32_t mode = (uint32_t)A.u.labels[0];
-    // In the modes that draw labels alone a drawn label replaces what the
-    // transfer function gives, so a sample outside the masks needs no density
-    // (labelled_at). Pre-integrated segments take every step's density.
-    const bool masks_first = mode >= 2u && !preintegrate;
     f3 v = -dir;
     f3 radiance = mk(0.0f);
     float transmittance = 1.0f;
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_cons
     bool has_grad = false, segment = false;
     if (state == MARCH) {
         tt = t.x + ign((float)px, (float)py) * step_mm;
-        if (!masks_first) prev_density = density_view(A, o_idx + d_idx * (tt - step_mm));
+        if (!MASKS_FIRST) prev_density = density_view(A, o_idx + d_idx * (tt - step_mm));
     }
     for (;;) {
         unsigned shading;
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS) k_dvr(const __grid_cons
                 tt += step_mm;
                 continue;
             }
-            if (masks_first) {
+            if (MASKS_FIRST) {
                 s = labelled_at<true>(A, idx, mode, grad, has_grad);
             } else {
                 // With smooth sampling the gradient comes with the density: a
@@ -745,8 +746,9 @@ cudaError_t launch_dvr(const PtArgs& a, const LightTex& shadow, const LightTex& 
     // x 400: 3.88 / 1.95 at 256^2, 4.54 / 3.52 at 512^2, 5.58 / 4.73 at 640^2, 6.53 /
     // 6.30 at 768^2, 9.20 / 10.27 at 1024^2; 256 x 256 x 200: 3.06 / 2.90 at 512^2,
     // 3.71 / 4.27 at 640^2. VV_DVR_LANES overrides (1, 2 or 4).
+    const bool masks = a.u.labels[0] >= 2.0f && a.u.lighting[2] == 0u;
     int lanes = 1;
-    if (a.u.labels[0] >= 2.0f && a.u.lighting[2] == 0u) {
+    if (masks) {
         lanes = (uint64_t)a.width * a.height < 3u << 17 ? 4 : 2;
         if (const char* e = std::getenv("VV_DVR_LANES")) lanes = std::atoi(e);
     }
@@ -754,8 +756,10 @@ cudaError_t launch_dvr(const PtArgs& a, const LightTex& shadow, const LightTex& 
         k_dvr_masks<4><<<dim3((a.width + 3) / 4, (a.height + 3) / 4), 64, 0, s>>>(a, shadow, ao);
     else if (lanes == 2)
         k_dvr_masks<2><<<dim3((a.width + 1) / 2, (a.height + 15) / 16), 64, 0, s>>>(a, shadow, ao);
+    else if (masks)
+        k_dvr<true><<<dim3((a.width + 7) / 8, (a.height + 7) / 8), 64, 0, s>>>(a, shadow, ao, dvr_gather(a));
     else
-        k_dvr<<<dim3((a.width + 7) / 8, (a.height + 7) / 8), 64, 0, s>>>(a, shadow, ao, dvr_gather(a));
+        k_dvr<false><<<dim3((a.width + 7) / 8, (a.height + 7) / 8), 64, 0, s>>>(a, shadow, ao, dvr_gather(a));
     return cudaGetLastError();
 }
 

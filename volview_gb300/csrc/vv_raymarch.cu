@@ -745,12 +745,16 @@ cudaError_t launch_dvr(const PtArgs& a, const LightTex& shadow, const LightTex& 
     // function modes). Two against four lanes, ms per frame, head/neck 512 x 512
     // x 400: 3.88 / 1.95 at 256^2, 4.54 / 3.52 at 512^2, 5.58 / 4.73 at 640^2, 6.53 /
     // 6.30 at 768^2, 9.20 / 10.27 at 1024^2; 256 x 256 x 200: 3.06 / 2.90 at 512^2,
-    // 3.71 / 4.27 at 640^2. VV_DVR_LANES overrides (1, 2 or 4).
+    // 3.71 / 4.27 at 640^2. The two are equal near 800^2 on the larger volume and
+    // near 550^2 on the smaller: the line lies between. VV_DVR_LANES overrides (1, 2 or 4; other
+    // values are ignored).
     const bool masks = a.u.labels[0] >= 2.0f && a.u.lighting[2] == 0u;
     int lanes = 1;
     if (masks) {
         lanes = (uint64_t)a.width * a.height < 3u << 17 ? 4 : 2;
-        if (const char* e = std::getenv("VV_DVR_LANES")) lanes = std::atoi(e);
+        const char* e = std::getenv("VV_DVR_LANES");
+        const int asked = e ? std::atoi(e) : 0;
+        if (asked == 1 || asked == 2 || asked == 4) lanes = asked;
     }
     if (lanes == 4)
         k_dvr_masks<4><<<dim3((a.width + 3) / 4, (a.height + 3) / 4), 64, 0, s>>>(a, shadow, ao);

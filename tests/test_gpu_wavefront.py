@@ -135,3 +135,25 @@ def test_flight_majorants_follow_their_inputs(small_cfg, gpu_ctx):
                 fresh.destroy()
     finally:
         kept.destroy()
+
+
+@pytest.mark.parametrize("samples", [1, 3])
+@pytest.mark.parametrize("size", [(37, 21), (131, 77), (311, 300)])
+def test_the_finishing_launch_changes_no_path(small_cfg, gpu_ctx, monkeypatch, size, samples):
+    """Paths handed to the finishing launch at the end, midway and all at once:
+    alone in their warps, and, where every warp is full with them (311 x 300), 32
+    to a warp."""
+    r = _renderer(small_cfg, gpu_ctx)
+    try:
+        p = _params(small_cfg, r)
+        p.path_tracing.samples_per_frame = samples
+        r.resize(*size)
+        images = []
+        for tail in ("0", "1024", "20000", "100000000"):
+            monkeypatch.setenv("VV_WF_TAIL", tail)
+            images.append(_frame(r, p))
+        for image in images[1:]:
+            for a, b in zip(image, images[0]):
+                assert np.array_equal(a, b)
+    finally:
+        r.destroy()

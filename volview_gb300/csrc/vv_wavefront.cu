@@ -890,7 +890,12 @@ __global__ void __launch_bounds__(256) k_wf_bin_place(const WfArgs W, const uint
 // their pixels' remaining samples and frames (a batched pass's from each path's
 // own request). Each runs alone in a warp, which takes the next one when it
 // ends: 32 divergent random walks to a warp take turns through each other's
-// code, and 2 or 4 to a warp finish no sooner.
+// code, and 2 or 4 to a warp finish no sooner. Only a remainder that gives every
+// warp 32 (the waves ran out with many samples per frame, or walks that outlast
+// them) is bound by throughput, and takes a lane each. A 512^2 frame of 256 x 256 x
+// 200 that hands over 4096, 16384, 65536, 262144 paths: 6.6, 11.5, 14.4, 21.3 ms
+// alone, 8.3, 13.3, 14.9, 17.9 with 32 to a warp; with 64 samples per frame 1163 and
+// 1126 ms. (2432 warps here: the line is at 77824 paths.)
 template <class X>
 __global__ void __launch_bounds__(128, 4) k_wf_finish(const __grid_constant__ X B, const WfArgs W, int cur) {
     chained();
@@ -899,7 +904,8 @@ __global__ void __launch_bounds__(128, 4) k_wf_finish(const __grid_constant__ X 
     uint32_t n_first = W.counts[WF_FIRST0 + cur], n = n_first + W.counts[cur];
     const Consts C0 = kernel_consts(B);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicSub(W.passes, 1u);
-    if ((threadIdx.x & 31u) != 0u) return;
+    const uint32_t lanes = n < gridDim.x * blockDim.x ? 1u : 32u;
+    if ((threadIdx.x & 31u) >= lanes) return;
     for (;;) {
         const uint32_t i = atomicAdd(&W.counts[WF_TAKE_EXT], 1u);  // zero: the last wave's shade cleared it
         if (i >= n) break;

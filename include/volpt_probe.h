@@ -56,6 +56,11 @@ vv_status vv_count_events(vv_renderer* r, int enable, uint64_t* out, size_t n);
  * and returns the summed milliseconds and the number of launches. */
 vv_status vv_time_pt(vv_renderer* r, int enable, double* ms, uint64_t* launches);
 
+/* Waits for the renderer's latest wavefront pass; then *passes = the passes of
+ * this process on its GPU now, *spread = whether that pass's last wave saw few
+ * enough there to spread its short queues over the whole chip. */
+vv_status vv_probe_company(vv_renderer* r, uint32_t* passes, uint32_t* spread);
+
 /* Light map importance sampling (pt.comp:204-233) from n random-stream states
  * seeds[n]: out[6n] = texel column, texel row, pdf, direction (xyz). Needs a
  * light map (vv_set_environment_map). */

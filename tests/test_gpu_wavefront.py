@@ -157,3 +157,41 @@ def test_the_finishing_launch_changes_no_path(small_cfg, gpu_ctx, monkeypatch, s
                 assert np.array_equal(a, b)
     finally:
         r.destroy()
+
+
+@pytest.mark.parametrize("beside", ["renderer", "engine"])
+def test_passes_beside_each_other_know_it_and_change_no_path(small_cfg, gpu_ctx, beside):
+    """A pass beside several of another renderer's, or of a batch engine's, packs
+    its short queues; the next one, by itself, spreads them. Both give the same
+    sums bit by bit, and no pass is left counted."""
+    r = _renderer(small_cfg, gpu_ctx)
+    ctx = R.Context(0)
+    other = _renderer(small_cfg, ctx)
+    engine = R.BatchEngine(ctx, 3, 16) if beside == "engine" else None
+    try:
+        p, q = _params(small_cfg, r), _params(small_cfg, other)
+        r.resize(131, 77)
+        other.resize(960, 720)  # three passes of 64 frames take many times as long as r's one
+        images, seen = [], []
+        for company in (True, False):
+            for k in range(3 if company else 0):
+                if engine:
+                    engine.record([(other, q, 1 + 64 * k, 64, True)])
+                else:
+                    other.record_frames(1 + 64 * k, 64, q)
+            r.reset_view()
+            r.record(1, p)
+            seen.append(r.probe_company())
+            images.append(r.read_accumulation())
+            other.synchronize()
+        assert [spread for _, spread in seen] == [False, True]
+        assert seen[0][0] >= 1 and seen[1][0] == 0
+        for a, b in zip(*images):
+            assert np.array_equal(a, b)
+    finally:
+        if engine:
+            engine.synchronize()
+            engine.destroy()
+        r.destroy()
+        other.destroy()
+        ctx.destroy()

@@ -119,6 +119,7 @@ struct vv_context {
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
     int sms = 0;
+    uint32_t* passes = nullptr;  // path-tracing passes on this GPU now (passes_on_device)
 };
 
 extern "C" vv_status vv_context_create_on_stream(int device, void* stream, vv_context** out) {
@@ -130,9 +131,12 @@ extern "C" vv_status vv_context_create_on_stream(int device, void* stream, vv_co
     CK(cudaSetDevice(device));
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    uint32_t* passes = nullptr;
+    CK(passes_on_device(&passes));
     vv_context* c = new vv_context();
     c->device = device;
     c->sms = sms;
+    c->passes = passes;
     if (stream) {
         c->stream = (cudaStream_t)stream;
     } else {
@@ -1361,10 +1365,6 @@ static PtArgs pt_args(vv_renderer* r, const UHead& u) {
     return a;
 }
 
-// Words of a renderer's `work` buffer: the single-kernel tracers' work counter and
-// status, then the passes on the device (WfArgs::passes).
-enum { WORK_PASSES = 16 };
-
 // The wavefront state of pass `P` for `cap` paths in flight on stream `s`:
 // its records, queues, counters and later-flight bins over volume `v`
 // (allocated when the pass needs more than it has).
@@ -1483,7 +1483,7 @@ static cudaError_t run_pt(vv_renderer* r, vv_renderer::Pass& P, PtArgs& a, cudaS
     WfArgs w;
     cudaError_t ce = wf_state(P, cap, r->vol, s, w);
     if (ce != cudaSuccess) return ce;
-    w.passes = r->work.as<uint32_t>() + WORK_PASSES;
+    w.passes = r->ctx->passes;
     return kernels_of(r).pt_wavefront(a, w, r->ctx->sms, s, launches);
 }
 
@@ -2009,9 +2009,7 @@ extern "C" vv_status vv_batch_create(vv_context* ctx, uint32_t passes, uint32_t 
         cudaError_t e = cudaStreamCreateWithFlags(&B.p.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&B.p.shown, cudaEventDisableTiming);
         if (e == cudaSuccess) e = B.p.counts.alloc(WF_COUNTERS * sizeof(uint32_t));
-        if (e == cudaSuccess) e = B.items.alloc((VV_BATCH_MAX + 1) * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMemsetAsync(B.items.p, 0, B.items.n, B.p.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(B.p.stream);  // passes on every stream count in pass 0's
+        if (e == cudaSuccess) e = B.items.alloc(VV_BATCH_MAX * sizeof(uint32_t));
         if (e == cudaSuccess) e = B.consts.alloc(VV_BATCH_MAX * WF_CONSTS_BYTES);
         if (e != cudaSuccess) {
             vv_batch_destroy(b);
@@ -2151,7 +2149,7 @@ extern "C" vv_status vv_batch_record(vv_batch* b, uint32_t n, vv_renderer* const
     WfArgs w;
     CK(wf_state(E.p, end, grid, s, w));
     w.items = E.items.as<uint32_t>();
-    w.passes = b->pass[0].items.as<uint32_t>() + VV_BATCH_MAX;
+    w.passes = b->ctx->passes;
     w.consts = E.consts.p;
     int launches = 0;
     CK(fmt0::launch_pt_wavefront_batch(B, w, b->ctx->sms, s, &launches));
@@ -2310,6 +2308,20 @@ extern "C" vv_status vv_time_pt(vv_renderer* r, int enable, double* ms, uint64_t
     if (ms) *ms = total;
     if (launches) *launches = r->pt_events.size();
     r->pt_events.clear();
+    return VV_OK;
+}
+
+// Waits for the renderer's latest pass.
+extern "C" vv_status vv_probe_company(vv_renderer* r, uint32_t* passes, uint32_t* spread) {
+    if (!r || !passes || !spread) return fail(VV_ERR_ARG, "null argument");
+    vv_status s = use_device(r);
+    if (s != VV_OK) return s;
+    vv_renderer::Pass& P = r->pass[(r->next_pass + r->passes - 1) % r->passes];
+    if (!P.slots.p) return fail(VV_ERR_STATE, "no wavefront pass has run");
+    CK(cudaStreamSynchronize(P.stream));
+    CK(cudaMemcpyAsync(spread, P.counts.as<uint32_t>() + WF_SPREAD, 4, cudaMemcpyDeviceToHost, P.stream));
+    CK(cudaMemcpyAsync(passes, r->ctx->passes, 4, cudaMemcpyDeviceToHost, P.stream));
+    CK(cudaStreamSynchronize(P.stream));
     return VV_OK;
 }
 

@@ -73,6 +73,10 @@ enum {
     COUNT_N = 10
 };
 
+// The current device's count of wavefront passes that have begun and not ended,
+// whichever renderer's or batch engine's.
+cudaError_t passes_on_device(uint32_t** count);
+
 cudaError_t launch_density(const int16_t* hu, void* out, const Vol& v, cudaStream_t s);
 cudaError_t launch_normals(const void* d, uint32_t* out, const Vol& v, const m3& w2i, cudaStream_t s);
 cudaError_t launch_masks(const MaskLaunch& L, cudaStream_t s, int* launches);
@@ -103,7 +107,7 @@ enum {
     WF_STOP = 13,     // 0 while waves run; 1 + the queue index the finishing launch takes over
     WF_MAP = 14,      // light map shadow rays queued by the key light's shadow rays
     WF_TAKE_MAP = 15, // entries of the light map shadow queue taken so far
-    WF_ALONE = 16,    // no other pass of this state's owner was on the device (shade looks, once per wave)
+    WF_SPREAD = 16,   // few passes are on the GPU: short queues go to all warps (shade looks, once per wave)
     WF_COUNTERS = 17
 };
 struct WfArgs {
@@ -134,7 +138,7 @@ struct WfArgs {
     int cell_shift;        // log2 of a cell's edge in voxels
     int cells_x, cells_y, cells_z;
     uint32_t bin_min;      // queues shorter than this are not ordered (the extend reads them as queued)
-    uint32_t* passes;      // passes of the state's owner (renderer or batch engine) on the device now
+    uint32_t* passes;      // this process's passes on the GPU now (passes_on_device)
     // Batched passes only: each request's next work item (VV_BATCH_MAX words)
     // and its constants derived from the uniforms (VV_BATCH_MAX records of
     // WF_CONSTS_BYTES), written by the pass's first launch.

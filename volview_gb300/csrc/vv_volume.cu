@@ -548,6 +548,11 @@ __global__ void k_brick_u8(const uint8_t* __restrict__ src, uint8_t* __restrict_
 
 static unsigned blocks_for(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// One word per device, in the library's own image: shared by all renderers and
+// engines of the process, and none of them has to outlive another's passes.
+__device__ uint32_t g_passes;
+cudaError_t passes_on_device(uint32_t** count) { return cudaGetSymbolAddress((void**)count, g_passes); }
+
 cudaError_t launch_density(const int16_t* hu, void* out, const Vol& v, cudaStream_t s) {
     k_density<<<blocks_for(vol_elems(v), 256), 256, 0, s>>>(hu, out, v);
     return cudaGetLastError();

@@ -387,21 +387,25 @@ __device__ void accumulate_items(const PtArgs& A, bool done, uint32_t item, cons
     atomicAdd(&A.normal[i], make_float4(v[8], v[9], v[10], v[11]));
 }
 
-constexpr uint32_t TAIL_ALONE = 2048u;
+constexpr uint32_t TAIL_SPREAD = 2048u, SPREAD_PASSES = 2u;
 // Lanes of each warp that take paths from a queue of n flights or shadow rays.
-// When no other pass of this state's owner is on the device, a short queue goes
-// to all warps of the launch, few lanes each: the divergent lanes of a warp take
-// turns, and a wave lasts as long as its slowest warp. Beside another pass the
-// same spreading takes issue slots that the other pass can use, so there every
-// warp takes 32. Measured (head/neck 1024^2): a frame alone 12.26 -> 11.07 ms and
-// overlapping frames 5.41 -> 5.43; spreading beside other passes too, 6.36. A
-// pass alone also leaves the waves earlier (TAIL_ALONE paths, 10.84 ms; 512, 1024
-// and 4096: 11.17, 11.07, 10.89). The count is looked at once per wave, between
-// its launches (WF_ALONE), so that all blocks of a launch see the same.
-__device__ __forceinline__ bool pass_alone(const WfArgs& W) { return W.counts[WF_ALONE] != 0u; }
+// With at most SPREAD_PASSES passes on the GPU, whichever renderers' they are, a
+// short queue goes to all warps of the launch, few lanes each: the divergent lanes
+// of a warp take turns, and a wave lasts as long as its slowest warp. With more
+// passes beside it the same spreading takes issue slots that they can use, so there
+// every warp takes 32. Measured (head/neck 1024^2): a frame alone 12.26 -> 11.07 ms
+// and overlapping frames 5.41 -> 5.43; spreading beside five other passes too, 6.36.
+// Renderers with one pass each, per frame, spreading while 1, 2, 3 passes or always:
+// two at 512^2 4.40, 4.04, 4.02, 4.01 ms, three 3.35, 3.36, 3.67, 3.55, four 2.81,
+// 2.80, 2.80, 3.47; at 1024^2 6.67, 6.25, 6.25, 6.24, then 5.42, 5.46, 5.55, 5.56 and
+// 4.97, 4.94, 4.96, 5.38. A spread pass also leaves the waves earlier (TAIL_SPREAD
+// paths, 10.84 ms; 512, 1024 and 4096: 11.17, 11.07, 10.89). The count is looked at
+// once per wave, between its launches (WF_SPREAD), so that all blocks of a launch
+// see the same.
+__device__ __forceinline__ bool pass_spreads(const WfArgs& W) { return W.counts[WF_SPREAD] != 0u; }
 __device__ __forceinline__ bool takes_paths(const WfArgs& W, uint32_t n) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t lanes = pass_alone(W) ? (n + warps - 1u) / warps : 32u;
+    const uint32_t lanes = pass_spreads(W) ? (n + warps - 1u) / warps : 32u;
     return (threadIdx.x & 31u) < lanes;
 }
 
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(256) k_wf_init(const __grid_constant__ X B, co
         for (int k = 0; k < WF_COUNTERS; k++) W.counts[k] = 0;
         W.counts[WF_FIRST0] = slots;
         W.counts[WF_ITEMS] = slots;
-        W.counts[WF_ALONE] = atomicAdd(W.passes, 1u) == 0u;
+        W.counts[WF_SPREAD] = atomicAdd(W.passes, 1u) < SPREAD_PASSES;
     }
     if constexpr (IsBatch<X>::value) {
         if (blockIdx.x == 0 && threadIdx.x < B.n) {
@@ -498,7 +502,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
         // Every block reads the same counts (nothing changes them before this
         // launch ends), so all blocks decide alike.
         uint32_t live = W.counts[WF_FIRST0 + cur] + W.counts[cur];
-        if (live <= (pass_alone(W) ? max(tail, TAIL_ALONE) : tail)) {
+        if (live <= (pass_spreads(W) ? max(tail, TAIL_SPREAD) : tail)) {
             if (blockIdx.x == 0 && threadIdx.x == 0) W.counts[WF_STOP] = (uint32_t)cur + 1u;
             return;
         }
@@ -631,7 +635,7 @@ __global__ void __launch_bounds__(128, VV_SHADE_MIN_BLOCKS) k_wf_shade(const __g
         W.counts[WF_TAKE_EXT] = 0;
         W.counts[WF_TAKE_FIRST] = 0;
         W.counts[WF_ESC0 + (cur ^ 1)] = 0;  // finished by the previous wave's scatter
-        W.counts[WF_ALONE] = *(volatile uint32_t*)W.passes <= 1u;
+        W.counts[WF_SPREAD] = *(volatile uint32_t*)W.passes <= SPREAD_PASSES;
     }
 }
 

@@ -76,6 +76,7 @@ PROBES = [
     ("vv_probe_extinction", C.c_int, [P, P, P, C.c_size_t, P, C.c_int, P]),
     ("vv_count_events", C.c_int, [P, C.c_int, P, C.c_size_t]),
     ("vv_time_pt", C.c_int, [P, C.c_int, P, P]),
+    ("vv_probe_company", C.c_int, [P, P, P]),
 ]
 
 # The learned denoiser's operators (include/volpt_nn.h).
@@ -322,6 +323,13 @@ class Renderer:
         fn = load().vv_probe_paths_exact if exact else load().vv_probe_paths
         check(fn(self.handle, C.byref(params), accumulated, _ptr(pix), pix.shape[0], _ptr(out)))
         return out
+
+    def probe_company(self):
+        """(passes on the GPU now, whether the latest pass's last wave spread its
+        short queues)."""
+        passes, spread = C.c_uint32(0), C.c_uint32(0)
+        check(load().vv_probe_company(self.handle, C.byref(passes), C.byref(spread)))
+        return passes.value, bool(spread.value)
 
     def time_pt(self, enable):
         """Starts (True) or stops (False -> (ms, launches)) timing the path-tracing launches."""

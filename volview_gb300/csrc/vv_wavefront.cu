@@ -942,10 +942,14 @@ __global__ void __launch_bounds__(128, 4) k_wf_finish(const __grid_constant__ X 
     }
 }
 
+// Lowers the count that k_wf_init raised, for a pass whose finishing launch could
+// not be queued.
+__global__ void k_wf_leave(const WfArgs W) { atomicSub(W.passes, 1u); }
+
 // A launch that may start its set-up before the launch before it has ended
 // (every kernel launched so begins with chained()).
 template <class... P, class... Q>
-static void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t s, Q... args) {
+static cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t s, const Q&... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)grid);
     config.blockDim = dim3((unsigned)block);
@@ -955,7 +959,7 @@ static void launch_chained(void (*kernel)(P...), int grid, int block, cudaStream
     early[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = early;
     config.numAttrs = 1;
-    cudaLaunchKernelEx(&config, kernel, P(args)...);
+    return cudaLaunchKernelEx(&config, kernel, P(args)...);
 }
 
 template <class K> static int blocks_per_sm(K kernel, int threads) {
@@ -981,7 +985,14 @@ static cudaError_t run_waves(const X& a, const WfArgs& w, int sms, cudaStream_t 
     const char* env = std::getenv("VV_WF_TAIL");
     uint32_t tail = env ? (uint32_t)std::atoi(env) : 1024u;
     k_wf_init<X><<<(slots + 255) / 256 < (uint32_t)(sms * 8) ? (slots + 255) / 256 : sms * 8, 256, 0, s>>>(a, w, slots);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     *launches += 1;
+    // From here the pass is counted on the GPU; the finishing launch lowers the count.
+    auto chain = [&](auto kernel, int grid, int block, const auto&... args) {
+        if (e == cudaSuccess) e = launch_chained(kernel, grid, block, s, args...);
+        if (e == cudaSuccess) *launches += 1;
+    };
     // All waves are queued at once, with no host round trip: the first launch
     // of each wave stops the waves on the device once at most `tail` paths
     // are left, the rest of the queued waves then return at once, and the
@@ -997,36 +1008,34 @@ static cudaError_t run_waves(const X& a, const WfArgs& w, int sms, cudaStream_t 
     const uint32_t first = base ? (uint32_t)std::max(1, std::atoi(base)) : 16u;
     int waves = (int)std::min<uint32_t>(first + 10u * rounds, 4096u);
     int cur = 0;
-    for (int wave = 0; wave < waves; wave++) {
+    for (int wave = 0; wave < waves && e == cudaSuccess; wave++) {
         // Launches that would find nothing to do are left out: first flights
         // after the first wave of a pass without refills, later flights in the
         // first wave, the ordering of queues that cannot reach bin_min.
         const bool first_flights = wave == 0 || refills;
-        if (first_flights) launch_chained(k_wf_extend<true, X>, g_ext, 128, s, a, w, cur, tail, 1);
-        if (wave > 0) launch_chained(k_wf_extend<false, X>, g_ext, 128, s, a, w, cur, tail, !first_flights);
-        launch_chained(k_wf_shade<X>, g_shade, 128, s, a, w, cur);
+        if (first_flights) chain(k_wf_extend<true, X>, g_ext, 128, a, w, cur, tail, 1);
+        if (wave > 0) chain(k_wf_extend<false, X>, g_ext, 128, a, w, cur, tail, !first_flights);
+        chain(k_wf_shade<X>, g_shade, 128, a, w, cur);
         if (map) {
-            launch_chained(k_wf_shadow<true, X>, g_shadow, 128, s, a, w);
-            launch_chained(k_wf_shadow_map<X>, g_shadow, 128, s, a, w);
-            *launches += 1;
+            chain(k_wf_shadow<true, X>, g_shadow, 128, a, w);
+            chain(k_wf_shadow_map<X>, g_shadow, 128, a, w);
         } else {
-            launch_chained(k_wf_shadow<false, X>, g_shadow, 128, s, a, w);
+            chain(k_wf_shadow<false, X>, g_shadow, 128, a, w);
         }
-        launch_chained(k_wf_scatter<X>, g_scatter, 128, s, a, w, cur);
-        *launches += 3 + first_flights + (wave > 0);
+        chain(k_wf_scatter<X>, g_scatter, 128, a, w, cur);
         cur ^= 1;
         if (slots < w.bin_min) continue;
         // The next wave's later flights, ordered by bin.
-        launch_chained(k_wf_bin_count, sms * 4, 256, s, w, w.ext_key[cur], cur);
-        launch_chained(k_wf_bin_scan, 1, 1024, s, w, cur);
-        launch_chained(k_wf_bin_place, sms * 4, 256, s, w, w.ext[cur], w.ext_key[cur], cur);
-        *launches += 3;
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        chain(k_wf_bin_count, sms * 4, 256, w, w.ext_key[cur], cur);
+        chain(k_wf_bin_scan, 1, 1024, w, cur);
+        chain(k_wf_bin_place, sms * 4, 256, w, w.ext[cur], w.ext_key[cur], cur);
     }
-    launch_chained(k_wf_finish<X>, g_finish, 128, s, a, w, cur);
-    *launches += 1;
-    return cudaGetLastError();
+    chain(k_wf_finish<X>, g_finish, 128, a, w, cur);
+    if (e != cudaSuccess) {
+        k_wf_leave<<<1, 1, 0, s>>>(w);
+        cudaGetLastError();
+    }
+    return e;
 }
 
 // Host side: one request's pass.

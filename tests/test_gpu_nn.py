@@ -400,3 +400,25 @@ def test_elementwise_gradients_at_vector_edges(lib, n, h, w, c):
         gd = dev(g, "half")
         assert lib.vv_nn_split(gd.data_ptr(), ca, c - ca, n * h * w, a.data_ptr(), b.data_ptr(), S) == 0
         assert np.array_equal(host(a), g[..., :ca]) and np.array_equal(host(b), g[..., ca:])
+
+
+@pytest.mark.parametrize("cin,cout", [(32, 32), (80, 32), (48, 48), (8, 96)])
+def test_weight_gradients_of_long_sums(lib, cin, cout):
+    """Sixteen 256 x 256 crops of non-negative values, a million products per
+    weight, against sums in 64 bits. Bar: a tensor-core sum of two steps of 16
+    products truncates by at most 17 + 1 units of 2^-23 relative, 2.2e-6; the
+    ordinary adds after it, up to 650 per weight over growing sums, err by about
+    2^-24 sqrt(650 / 3) / sqrt(3) = 5e-7 (one sigma), 2.5e-6 at five."""
+    n, h, w = 16, 256, 256
+    torch.manual_seed(cin + cout)
+    x = torch.rand((n, h, w, cin), device="cuda").half()
+    dy = torch.rand((n, h, w, cout), device="cuda").half()
+    dw = torch.zeros((cout, 9, cin), device="cuda")
+    assert lib.vv_nn_conv3x3_wgrad(x.data_ptr(), dy.data_ptr(), n, h, w, cin, cout, dw.data_ptr(), S) == 0
+    ref = torch.zeros((cout, 9, cin), dtype=torch.float64, device="cuda")
+    for img in range(n):
+        xp = torch.nn.functional.pad(x[img].double(), (0, 0, 1, 1, 1, 1))
+        d = dy[img].double().reshape(-1, cout).T
+        for tap in range(9):
+            ref[:, tap] += d @ xp[tap // 3:tap // 3 + h, tap % 3:tap % 3 + w].reshape(-1, cin)
+    assert float(((dw.double() - ref) / ref).abs().max()) <= 4.7e-6

@@ -214,16 +214,23 @@ __device__ __forceinline__ void ldmatrix_t(uint32_t r[4], uint32_t addr) {
 // and four rows that cp.async fills one row ahead; both fragments come from
 // ldmatrix.trans (the reduction runs over pixels, the rows of both tiles), a
 // tap's x fragments `tap % 3` pixels further on. Row pitches are odd multiples
-// of 16 bytes, so the eight rows of a matrix fall in distinct banks. One FP32
-// add per weight and block at the end. Bound by shared memory and the legacy
-// tensor path; the kernel above (2-byte strided loads straight into fragments,
-// a chunk of 256 pixels per warp) took 1 718 us for the U-Net's 19 layers on
-// four 256 x 256 crops, this one 428 us (the largest, 80 -> 32: 332 -> 55).
+// of 16 bytes, so the eight rows of a matrix fall in distinct banks. The tensor
+// core's adds truncate, and a run is up to 1024 steps of 16 pixels, so only CHAIN
+// steps are summed there; ordinary FP32 adds, rounded to nearest, take each such sum
+// into the accumulators (a whole run in the tensor core drifted by 5e-6 relative on
+// four 256 x 256 crops of same-sign values, 1e-4 on 64; this way by 1e-7 on either,
+// the kernel above by 1e-6). One FP32 add per weight and block at the end. Bound by
+// shared memory, the legacy tensor path and those adds; on four 256 x 256 crops the
+// kernel above (2-byte strided loads straight into fragments, a chunk of 256 pixels
+// per warp) takes 321 us for 80 -> 32 channels and 1330 for 96 -> 96, this one 64 and
+// 232, and would take 54 and 210 without the adds. Chains of 1, 2, 4 steps: 69, 64,
+// 72 us and (3 x 3 tiles) 232, 244, 248.
 template <int MT, int CT>
 __global__ void __launch_bounds__(288, MT * CT > 6 ? 1 : 2) k_wgrad_tile(const __half* __restrict__ x, const __half* __restrict__ dy,
                                                        int h, int w, int cin, int cout, int seg, int run,
                                                        int co_tiles, float* __restrict__ dw) {
     constexpr int XP = CT * 16 + 8, DP = MT * 16 + 8;  // row pitches, in halves
+    constexpr int CHAIN = MT * CT > 6 ? 1 : 2;         // steps of 16 pixels per tensor-core sum
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t xs = smem_addr(smem), x_row = (uint32_t)(seg + 2) * XP * 2;
     const uint32_t ds = xs + 4 * x_row, d_row = (uint32_t)seg * DP * 2;
@@ -275,19 +282,35 @@ __global__ void __launch_bounds__(288, MT * CT > 6 ? 1 : 2) k_wgrad_tile(const _
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
         const uint32_t a_row = ds + (i & 1) * d_row + a_off, b_row = xs + ((i + tap / 3) & 3) * x_row + b_off;
-        for (int k = 0; k < seg; k += 16) {
-            uint32_t a[MT][4];
+        for (int k = 0; k < seg; k += 16 * CHAIN) {
+            uint32_t a[CHAIN][MT][4];
 #pragma unroll
-            for (int m = 0; m < MT; m++) ldmatrix_t(a[m], a_row + (k * DP + m * 16) * 2);
+            for (int q = 0; q < CHAIN; q++)
+                if (q == 0 || k + 16 * q < seg)
+#pragma unroll
+                    for (int m = 0; m < MT; m++) ldmatrix_t(a[q][m], a_row + ((k + 16 * q) * DP + m * 16) * 2);
 #pragma unroll
             for (int j = 0; j < CT; j++) {
-                uint32_t b[4];
-                ldmatrix_t(b, b_row + (k * XP + j * 16) * 2);
+                float d[MT][2][4];
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    mma16816(acc[m][2 * j], a[m], b);
-                    mma16816(acc[m][2 * j + 1], a[m], b + 2);
-                }
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) d[m][e >> 2][e & 3] = 0.0f;
+#pragma unroll
+                for (int q = 0; q < CHAIN; q++)
+                    if (q == 0 || k + 16 * q < seg) {
+                        uint32_t b[4];
+                        ldmatrix_t(b, b_row + ((k + 16 * q) * XP + j * 16) * 2);
+#pragma unroll
+                        for (int m = 0; m < MT; m++) {
+                            mma16816(d[m][0], a[q][m], b);
+                            mma16816(d[m][1], a[q][m], b + 2);
+                        }
+                    }
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) acc[m][2 * j + (e >> 2)][e & 3] += d[m][e >> 2][e & 3];
             }
         }
         __syncthreads();

@@ -422,3 +422,23 @@ def test_weight_gradients_of_long_sums(lib, cin, cout):
         for tap in range(9):
             ref[:, tap] += d @ xp[tap // 3:tap // 3 + h, tap % 3:tap % 3 + w].reshape(-1, cin)
     assert float(((dw.double() - ref) / ref).abs().max()) <= 4.7e-6
+
+
+def test_weight_gradients_of_more_channels_than_tiles_fit_a_grid(lib):
+    """3.2 million input channels (100000 tiles of 32): one row of 16 pixels, so
+    the three taps of that row are sums of up to 16 products of small integers,
+    exact, and the others 0."""
+    n, h, w, cin, cout = 1, 1, 16, 3200000, 8
+    x = torch.randint(-2, 3, (w, cin), device="cuda").half()
+    dy = torch.randint(-2, 3, (w, cout), device="cuda").half()
+    dw = torch.zeros((cout, 9, cin), device="cuda")
+    assert lib.vv_nn_conv3x3_wgrad(x.data_ptr(), dy.data_ptr(), n, h, w, cin, cout, dw.data_ptr(), S) == 0
+    torch.cuda.synchronize()
+    for tap in range(9):
+        if tap // 3 != 1:
+            assert not dw[:, tap].any()
+            continue
+        dx = tap % 3 - 1
+        lo, hi = max(0, -dx), min(w, w - dx)
+        ref = dy[lo:hi].float().T @ x[lo + dx:hi + dx].float()
+        assert torch.equal(dw[:, tap], ref)

@@ -815,6 +815,7 @@ static int wgrad_tile(int c) {
     const int pad3 = (units + 2) / 3 * 3, pad2 = (units + 1) / 2 * 2;
     return pad3 <= pad2 ? 3 : 2;
 }
+static long wgrad_tiles(int c) { return (c + wgrad_tile(c) * 16L - 1) / (wgrad_tile(c) * 16L); }
 template <int MT, int CT>
 static vv_status launch_wgrad(const __half* x, const __half* dy, int n, int h, int w, int cin, int cout, float* dw,
                               cudaStream_t s) {
@@ -828,7 +829,6 @@ static vv_status launch_wgrad(const __half* x, const __half* dy, int n, int h, i
     const int run = (int)((h + per_column - 1) / per_column);
     const long grid = columns * ((h + run - 1) / run);
     const size_t smem = ((size_t)4 * (seg + 2) * (CT * 16 + 8) + (size_t)2 * seg * (MT * 16 + 8)) * 2;
-    if (grid > 0x7fffffffL) return VV_ERR_ARG;
     k_wgrad_tile<MT, CT><<<dim3((unsigned)grid, tiles), 288, smem, s>>>(x, dy, h, w, cin, cout, seg, run, co_tiles, dw);
     return launched();
 }
@@ -838,7 +838,9 @@ extern "C" vv_status vv_nn_conv3x3_wgrad(const void* x, const void* dy, int n, i
     if (!x || !dy || !dw || n <= 0 || h <= 0 || w <= 0 || w % 16 || cin <= 0 || cin % 8 || cout <= 0 || cout % 8)
         return VV_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    if (aligned16(x) && aligned16(dy)) {
+    // A grid's second dimension holds at most 65535 tiles of channels; wider layers
+    // run on the kernel of 16 x 64 channels, as unaligned tensors do.
+    if (aligned16(x) && aligned16(dy) && wgrad_tiles(cout) * wgrad_tiles(cin) <= 65535) {
         const __half *X = (const __half*)x, *D = (const __half*)dy;
         switch (wgrad_tile(cout) * 4 + wgrad_tile(cin)) {
             case 1 * 4 + 1: return launch_wgrad<1, 1>(X, D, n, h, w, cin, cout, dw, s);

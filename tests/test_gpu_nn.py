@@ -442,3 +442,13 @@ def test_weight_gradients_of_more_channels_than_tiles_fit_a_grid(lib):
         lo, hi = max(0, -dx), min(w, w - dx)
         ref = dy[lo:hi].float().T @ x[lo + dx:hi + dx].float()
         assert torch.equal(dw[:, tap], ref)
+
+
+@pytest.mark.parametrize("pixels", [63, 129, 40001])
+@pytest.mark.parametrize("c", [8, 96, 176, 512, 1024])
+def test_bias_gradients_of_any_width(lib, pixels, c):
+    """Sums of small integers, exact in FP32 whatever the blocks' share."""
+    dy = torch.randint(-3, 4, (pixels, c), device="cuda").half()
+    db = torch.zeros(c, device="cuda")
+    assert lib.vv_nn_bias_grad(dy.data_ptr(), pixels, c, db.data_ptr(), S) == 0
+    assert torch.equal(db, dy.double().sum(0).float())

@@ -1299,17 +1299,11 @@ __device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F,
     return clip_depth(A, origin + F.d_idx * F.tt, plane) <= 0.0f ? FF_SAMPLE : FF_CONTINUE;
 }
 // The rest of that iteration: the collision at F.tt, accepted (FF_HIT) or null.
-// ff_fetch leaves its sample and returns the extinction there, a ghost's before
-// its shell's scale (ghost_shell); ff_collide decides on the extinction.
-__device__ __forceinline__ float ff_fetch(const PtArgs& A, f3 origin, bool smooth, const Flight& F, f3& idx, Sample& s,
-                                          int& cap_plane, float& cut) {
+__device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
+                                         const Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
     idx = origin + F.d_idx * F.tt;
     cut = clip_depth(A, idx, cap_plane);
-    s = sample_labels<true>(A, idx, smooth && A.u.env[1] > 0.5f);
-    return s.extinction;
-}
-__device__ __forceinline__ int ff_collide(const PtArgs& A, float ext, int hero, f3& spectral, const Flight& F,
-                                          const Sample& s, Rng& rng) {
+    float ext = extinction_unclipped(A, idx, dir, smooth, s, cap_plane, cut);
     if (ext <= 0.0f) return FF_CONTINUE;
     f3 sigma = path_sigma(A, s, ext);
     float sh = comp(sigma, hero);
@@ -1319,12 +1313,6 @@ __device__ __forceinline__ int ff_collide(const PtArgs& A, float ext, int hero, 
     }
     spectral *= gmax(F.maj - sigma, 0.0f) / (F.maj - sh);
     return FF_CONTINUE;
-}
-__device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral,
-                                         const Flight& F, f3& idx, Sample& s, int& cap_plane, float& cut, Rng& rng) {
-    float ext = ff_fetch(A, origin, smooth, F, idx, s, cap_plane, cut);
-    if (s.ghost && ext > 0.0f) ext *= ghost_shell(A, idx, s, -dir, cap_plane, cut);
-    return ff_collide(A, ext, hero, spectral, F, s, rng);
 }
 
 __device__ bool free_flight(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral, f3& idx,

@@ -195,3 +195,28 @@ def test_passes_beside_each_other_know_it_and_change_no_path(small_cfg, gpu_ctx,
         r.destroy()
         other.destroy()
         ctx.destroy()
+
+
+@pytest.mark.parametrize("kernel", ["wavefront", "persistent"])
+def test_majorants_are_counted_once_per_brick_that_a_flight_enters(gpu_ctx, monkeypatch, kernel):
+    """One dense brick, clipped away whole: a flight crosses it through many
+    tentative collisions, none of which reads a voxel or casts a shadow ray, and
+    the one majorant it needs is one event."""
+    if kernel != "wavefront":
+        monkeypatch.setenv("VV_PT_KERNEL", kernel)
+    hu = np.full((8, 8, 8), 1500, np.int16)
+    r = R.Renderer(gpu_ctx, abi.volume_struct(hu, (4.0, 4.0, 4.0)), abi.tf_struct(abi.PRESETS["bone"]))
+    try:
+        p = scene.frame_params_for(dict(min_spacing=4.0, label_params=abi.label_params_default()), list(r.center),
+                                   r.diagonal, clip_sagittal=True)
+        p.clipping.planes[0].position = abi.f32(r.bounds[0][0] - 1.0)
+        p.camera.distance = abi.f32(p.camera.distance * 0.5)
+        p.path_tracing.denoiser = abi.DENOISE_OFF
+        r.resize(40, 30)
+        r.count_events(True)
+        r.record(1, p)
+        events = r.count_events(False)
+        assert events["path"] == 1200 and events["trilinear"] == events["cubic"] == 0
+        assert 600 <= events["majorant"] <= 1200
+    finally:
+        r.destroy()

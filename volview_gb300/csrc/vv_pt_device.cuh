@@ -1165,10 +1165,7 @@ __device__ __forceinline__ f3 event_albedo(const PtArgs& A, const Sample& s) {
 }
 // flight_majorant (pt.comp:157-163) of brick `b` (brick_index), from the grid
 // prepared for the frame's uniforms.
-__device__ __forceinline__ float flight_majorant_of(const PtArgs& A, int b) {
-    if (A.u.path[3] != 0u) count(A, COUNT_MAJORANT);
-    return __ldg(A.flight + b);
-}
+__device__ __forceinline__ float flight_majorant_of(const PtArgs& A, int b) { return __ldg(A.flight + b); }
 __device__ __forceinline__ float phase_hg(const PtArgs& A, float cos_t) {
     float g = A.u.env[2];
     float d = 1.0f + g * g - 2.0f * g * cos_t;
@@ -1263,13 +1260,20 @@ struct Flight {
 };
 enum { FF_CONTINUE = 0, FF_HIT = 1, FF_ESCAPE = 2, FF_SAMPLE = 4 };
 
-__device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Flight& F) {
+// The brick that a flight's last counted majorant was of, while events are counted:
+// a flight needs one per brick that it enters, although it reads one at every
+// advance. Volatile, so that it lies in local memory and takes no register from the
+// flight.
+typedef volatile int CountedBrick;
+
+__device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Flight& F, CountedBrick& counted) {
     F.d_idx = mul(w2i3(A), dir);
     float2 tr = intersect_volume(A, origin, F.d_idx);
     F.inv_d = brick_inv_dir(F.d_idx);
     F.tt = tr.x;
     F.t_end = tr.y;
     F.iter = 0;
+    if (A.counters) counted = -1;
 }
 
 // One iteration of pt.comp:307-333 up to the voxel fetch. FF_CONTINUE: an
@@ -1279,10 +1283,15 @@ __device__ __forceinline__ void ff_begin(const PtArgs& A, f3 origin, f3 dir, Fli
 // The majorant is fetched at every advance: from the prepared grid that is
 // cheaper than looking whether the brick has changed (711 M path samples/s against
 // 705; 685 when every fetch applied the uniforms).
-__device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F, Rng& rng) {
+__device__ __forceinline__ int ff_advance(const PtArgs& A, f3 origin, Flight& F, CountedBrick& counted, Rng& rng) {
     if (!(F.iter < 4096 && F.tt < F.t_end)) return FF_ESCAPE;
     f3 p = origin + F.d_idx * F.tt;
-    F.maj = flight_majorant_of(A, brick_index(A, p));
+    const int b = brick_index(A, p);
+    if (A.counters && A.u.path[3] != 0u && counted != b) {
+        counted = b;
+        count(A, COUNT_MAJORANT);
+    }
+    F.maj = flight_majorant_of(A, b);
     F.iter++;
     float exit = F.tt + brick_exit(p, F.inv_d, far_planes(F.inv_d)) + 1e-3f;
     if (F.maj <= 0.0f) {
@@ -1318,9 +1327,10 @@ __device__ __forceinline__ int ff_sample(const PtArgs& A, f3 origin, f3 dir, boo
 __device__ bool free_flight(const PtArgs& A, f3 origin, f3 dir, bool smooth, int hero, f3& spectral, f3& idx,
                             Sample& s, int& cap_plane, float& cut, Rng& rng) {
     Flight F;
-    ff_begin(A, origin, dir, F);
+    CountedBrick counted;
+    ff_begin(A, origin, dir, F, counted);
     for (;;) {
-        int r = ff_advance(A, origin, F, rng);
+        int r = ff_advance(A, origin, F, counted, rng);
         if (r == FF_SAMPLE) r = ff_sample(A, origin, dir, smooth, hero, spectral, F, idx, s, cap_plane, cut, rng);
         if (r == FF_HIT) return true;
         if (r == FF_ESCAPE) return false;
@@ -1362,6 +1372,7 @@ __device__ __forceinline__ int tr_advance(const PtArgs& A, f3 origin, Shadow& T,
         T.result *= 0.1f / peak;
     }
     f3 p = origin + T.d_idx * T.tt;
+    if (A.u.path[3] != 0u) count(A, COUNT_MAJORANT);
     T.maj = flight_majorant_of(A, brick_index(A, p));
     float exit = T.tt + brick_exit(p, T.inv_d, far_planes(T.inv_d)) + 1e-3f;
     if (T.maj <= 0.0f) {

@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
     Rng rng;
     uint32_t word = 0;  // P2.w: volumes, sample, hero
     Flight F;
+    CountedBrick counted;
     Vertex V;
     for (;;) {
         const uint32_t k = take_item(taken, n, takes);
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
             uint32_t surfaces = ubits(b.w) >> 16, volumes = word & 1023u;
             if (surfaces <= C.max_bounces && volumes <= C.volume_limit) {
                 count(A, COUNT_VERTEX);
-                ff_begin(A, origin, dir, F);
+                ff_begin(A, origin, dir, F, counted);
                 state = LANE_ADVANCE;
             }
         }
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(128, VV_EXTEND_MIN_BLOCKS)
 #pragma unroll 1
                 for (int twice = 0; twice < 2; twice++) {  // one look at the warp per two advances
                     if (state != LANE_ADVANCE) continue;
-                    const int res = ff_advance(args_of(B, r), origin, F, rng);
+                    const int res = ff_advance(args_of(B, r), origin, F, counted, rng);
                     if (res == FF_SAMPLE) state = LANE_SAMPLE;
                     if (res == FF_ESCAPE) {
                         state = LANE_OUT;

@@ -2,6 +2,8 @@
 dimensions are not multiples of the 8^3 bricks (ragged bricks, anisotropic
 spacing) rendered at an odd image size, labels that draw nothing, and the
 size limits of the C ABI. Tolerances as in test_gpu_parity.py."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -118,3 +120,36 @@ def test_size_limits(small_cfg, gpu_ctx):
     r.record(1, p)
     assert r.read_output().shape == (1, 1, 4)
     r.destroy()
+
+
+def test_denoiser_next_to_a_depth_that_is_not_a_number(small_cfg, gpu_ctx):
+    """A pixel whose accumulated depth is NaN poisons the taps of the pixels
+    around it, background ones too, as in the shader: their weights' sum is NaN and
+    they stay unfiltered. Against the oracle on the same buffers; the noise is
+    +-50 %, the bar the last bits of expf and powf through five levels."""
+    torch = pytest.importorskip("torch")
+    W, H, n = 64, 48, 4
+    rng = np.random.default_rng(3)
+    accum = np.zeros((H, W, 4), np.float32)
+    accum[..., :3] = rng.uniform(0.5, 1.5, (H, W, 3)) * n
+    albedo = np.full((H, W, 4), 0.7 * n, np.float32)
+    albedo[..., 3] = 1.3 * n
+    normal = np.zeros((H, W, 4), np.float32)
+    normal[..., 3] = 1e4 * n           # background
+    normal[:, 20:, 2] = n              # a wall
+    normal[:, 20:, 3] = 100.0 * n
+    normal[24, 21, 3] = np.nan
+    cpu = O.CpuRenderer(small_cfg["volume"], small_cfg["tf"], small_cfg["hu"])
+    cpu.resize(W, H)
+    cpu.accum, cpu.albedo, cpu.normal, cpu.accumulated = accum, albedo, normal, n
+    p = scene.frame_params_for(small_cfg, list(cpu.geo.center), cpu.geo.diagonal)
+    ref = cpu.denoise(p).view(np.float16).astype(np.float32)[..., :3]
+    bufs = [torch.from_numpy(a).cuda() for a in (accum, albedo, normal)]
+    out = torch.zeros((H, W, 4), dtype=torch.int16, device="cuda")
+    R.check(R.load().vv_denoise_atrous_noalloc(*(C.c_void_p(b.data_ptr()) for b in bufs), C.c_void_p(out.data_ptr()),
+                                               W, H, n, None))
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().view(np.float16).astype(np.float32)[..., :3]
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref))
+    ok = np.isfinite(ref)
+    assert np.all(np.abs(got - ref)[ok] <= 0.01 * np.abs(ref)[ok])

@@ -83,9 +83,9 @@ __global__ void __launch_bounds__(256) k_denoise_prepare(const PostArgs a) {
 // denoise.comp:96-144: one a-trous level, 5x5 B3 taps `step` pixels apart. Bound
 // by instruction issue (a power, three exponentials and three divisions per
 // tap). A tap between a pixel with a normal and one without has weight 0, which
-// adds nothing (its value is checked finite: 0 times an infinity would), and
-// between two without the normals' power is not needed: background pixels
-// skip it (246 -> 198 us at 1024^2).
+// adds nothing (its value and depth are checked finite: 0 times an infinity or a
+// NaN would; a NaN albedo makes the value one), and between two without the
+// normals' power is not needed: background pixels skip it (246 -> 198 us at 1024^2).
 __global__ void __launch_bounds__(256) k_denoise_level(const PostArgs a, int step, int from_pong) {
     int x = blockIdx.x * 16 + threadIdx.x % 16, y = blockIdx.y * 16 + threadIdx.x / 16;
     int W = (int)a.width, H = (int)a.height;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(256) k_denoise_level(const PostArgs a, int ste
             float w_normal = 1.0f;
             if (center_flat || q_flat) {
                 if (!(center_flat && q_flat)) {
-                    if (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + fabsf(c.w) < INFINITY) continue;
+                    if (fabsf(c.x) + fabsf(c.y) + fabsf(c.z) + fabsf(c.w) + fabsf(g.w) < INFINITY) continue;
                     w_normal = 0.0f;
                 }
             } else {

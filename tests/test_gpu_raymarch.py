@@ -255,3 +255,28 @@ def test_transfer_function_alone_as_with_labels_that_draw_nothing(small_cfg, gpu
         assert np.array_equal(images[0], images[1])
     finally:
         r.destroy()
+
+
+def test_lanes_per_ray_light_an_extinction_that_is_not_a_number(small_cfg, gpu_ctx, monkeypatch):
+    """A label extinction of NaN shows as NaN pixels, with two and four lanes per
+    ray as with one."""
+    cfg = small_cfg
+    r = R.Renderer(gpu_ctx, cfg["volume"], cfg["tf"])
+    try:
+        r.set_labels(cfg["labels_vol"], abi.soft_struct(cfg["soft"]))
+        p = scene.frame_params_for(cfg, list(r.center), r.diagonal)
+        p.camera.distance = abi.f32(p.camera.distance * 0.45)
+        p.path_tracing.enabled = 0
+        p.labels.extinction = float("nan")
+        r.resize(37, 21)
+        images = []
+        for lanes in ("1", "2", "4"):
+            monkeypatch.setenv("VV_DVR_LANES", lanes)
+            r.reset_view()
+            r.record(1, p)
+            images.append(r.read_hdr())
+        assert np.isnan(_half(images[0])).any()
+        for image in images[1:]:
+            assert np.array_equal(np.isnan(_half(image)), np.isnan(_half(images[0])))
+    finally:
+        r.destroy()

@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(64, VV_DVR_MIN_BLOCKS)
             }
             if (mine) {
                 s = labelled_at<true>(A, idx, mode, grad, has_grad);
-                lit = s.extinction > 0.0f;
+                lit = !(s.extinction <= 0.0f);
             }
             if (found == 0) marching = false;
         }

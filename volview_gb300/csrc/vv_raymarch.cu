@@ -152,11 +152,10 @@ __device__ __forceinline__ float ign(float px, float py) {
 // texels, so it may also weigh the slice being written, by up to 1e-5: those texels
 // count as 0, as they are before the launch, and not as whatever other threads
 // have written by then.
-// CHAINED: the launch that writes the texels read here may still have been
-// running when the reading one started, so the read-only path, which is for data
-// that does not change while a kernel lives, is not for them. The loads are
-// coherent ones from L2, since L1 may hold a sector from before (with x as the
-// sweep's axis one sector holds texels of several slices).
+// CHAINED: the launch that writes the texels read here may not have ended when the
+// reading one started, so the read-only path, which is for data that does not
+// change while a kernel lives, is not for them; the loads are ordinary ones, after
+// the wait for that launch.
 struct LightVol {
     const ushort4* data;  // RGBA16F, x fastest
     int w, h, d, axis, slice;
@@ -165,7 +164,7 @@ template <bool CHAINED> __device__ __forceinline__ float4 lv_texel(const LightVo
     if (x < 0 || y < 0 || z < 0 || x >= v.w || y >= v.h || z >= v.d) return make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     if ((v.axis == 0 ? x : v.axis == 1 ? y : z) == v.slice) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     long i = ((long)z * v.h + y) * v.w + x;
-    ushort4 t = CHAINED ? __ldcg(v.data + i) : __ldg(v.data + i);
+    ushort4 t = CHAINED ? v.data[i] : __ldg(v.data + i);
     return make_float4(h2f(t.x), h2f(t.y), h2f(t.z), h2f(t.w));
 }
 template <bool CHAINED> __device__ float4 lv_linear(const LightVol& v, f3 tc) {
@@ -378,9 +377,10 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     const ShadowSweep w = shadow_sweep_of(A, sx, sy, sz, axis);
     const long at = ((long)p[2] * sy + p[1]) * sx + p[0];
     f3 here = mk((float)p[0], (float)p[1], (float)p[2]);
-    // The next slice's launch is prepared behind this one; it, too, waits for the
-    // slice before it (and so for all) past this point.
-    if (GIVEN) asm volatile("griddepcontrol.launch_dependents;");
+    // A chained launch's set-up overlaps the slice before it, whose end (and so that
+    // of all before) it waits for here. Its blocks come once that slice's have ended:
+    // let in earlier (launch_dependents), they would have to read past L1, which may
+    // hold sectors from before, and cost more than they gain (below).
     const float4 f = GIVEN ? __ldg(factors + at) : shadow_factors(A, w, here);
     if (GIVEN) asm volatile("griddepcontrol.wait;" ::: "memory");
     f3 prev = here + w.l_idx * w.s;
@@ -687,7 +687,9 @@ cudaError_t launch_shadow_sweep(const PtArgs& a, ushort4* vol, int sx, int sy, i
     for (int i = 0; i < n; i++) {
         int slice = sign > 0 ? n - 1 - i : i;
         if (factors) {
-            // Programmatic dependent launch: 6.7 -> 5.0 us per slice.
+            // Programmatic dependent launch. A sweep of 126 x 122 x 94 texels along x, y,
+            // z: 1.14, 0.78, 0.77 ms; with launch_dependents and loads from L2 1.82,
+            // 1.04, 1.14; plain launches that take the factors themselves 2.13, 1.99, 1.88.
             cudaLaunchConfig_t config = {};
             config.gridDim = g;
             config.blockDim = dim3(64);

@@ -161,27 +161,32 @@ struct LightVol {
     int w, h, d, axis, slice;
 };
 template <bool CHAINED> __device__ __forceinline__ float4 lv_texel(const LightVol& v, int x, int y, int z) {
-    if (x < 0 || y < 0 || z < 0 || x >= v.w || y >= v.h || z >= v.d) return make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    if ((v.axis == 0 ? x : v.axis == 1 ? y : z) == v.slice) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    long i = ((long)z * v.h + y) * v.w + x;
-    ushort4 t = CHAINED ? v.data[i] : __ldg(v.data + i);
+    const bool out = x < 0 || y < 0 || z < 0 || x >= v.w || y >= v.h || z >= v.d;
+    const bool own = (v.axis == 0 ? x : v.axis == 1 ? y : z) == v.slice;
+    const uint16_t none = out ? 0x3c00 : 0;  // 1 or 0
+    ushort4 t = make_ushort4(none, none, none, none);
+    if (!out && !own) {
+        const ushort4* at = v.data + ((long)z * v.h + y) * v.w + x;
+        t = CHAINED ? *at : __ldg(at);
+    }
     return make_float4(h2f(t.x), h2f(t.y), h2f(t.z), h2f(t.w));
 }
-template <bool CHAINED> __device__ float4 lv_linear(const LightVol& v, f3 tc) {
+template <bool CHAINED> __device__ __forceinline__ float4 lv_linear(const LightVol& v, f3 tc) {
     float x = tc.x * (float)v.w - 0.5f, y = tc.y * (float)v.h - 0.5f, z = tc.z * (float)v.d - 0.5f;
     int i0 = (int)floorf(x), j0 = (int)floorf(y), k0 = (int)floorf(z);
     float a = x - (float)i0, b = y - (float)j0, c = z - (float)k0;
+    float4 t[8];  // all loads before the sums: a slice is one chain of latencies
+#pragma unroll
+    for (int k = 0; k < 8; k++) t[k] = lv_texel<CHAINED>(v, i0 + (k & 1), j0 + ((k >> 1) & 1), k0 + (k >> 2));
     float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int dk = 0; dk < 2; dk++)
-        for (int dj = 0; dj < 2; dj++)
-            for (int di = 0; di < 2; di++) {
-                float w = (di ? a : 1.0f - a) * (dj ? b : 1.0f - b) * (dk ? c : 1.0f - c);
-                float4 t = lv_texel<CHAINED>(v, i0 + di, j0 + dj, k0 + dk);
-                r.x += t.x * w;
-                r.y += t.y * w;
-                r.z += t.z * w;
-                r.w += t.w * w;
-            }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        float w = (k & 1 ? a : 1.0f - a) * (k & 2 ? b : 1.0f - b) * (k & 4 ? c : 1.0f - c);
+        r.x += t[k].x * w;
+        r.y += t[k].y * w;
+        r.z += t[k].z * w;
+        r.w += t[k].w * w;
+    }
     return r;
 }
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
@@ -360,8 +365,10 @@ __global__ void __launch_bounds__(128) k_shadow_factors(const __grid_constant__ 
 // slice before it, in five linear lookups, times the factors (from `factors`,
 // or taken here where the caller has no room for them). The slices are a chain
 // of dependent launches, so what is not part of the chain is kept out of it.
-// Measured on 301 x 255 x 203 voxels: 17.5 -> 6.7 us per slice (151 of them) and 43 us
-// for the factors.
+// Measured on 301 x 255 x 203 voxels: factors in the slices 17.5 us for each of 151;
+// ahead of them 43 us in all. The loads of a lookup are unconditional but for their
+// predicates, so that they overlap (with a branch per texel the sweep below took
+// 1.12, 1.14, 0.78, 0.76 ms).
 template <bool GIVEN>
 __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtArgs A, ushort4* __restrict__ vol,
                                                      const float4* __restrict__ factors, int sx, int sy, int sz,
@@ -390,12 +397,14 @@ __global__ void __launch_bounds__(64) k_shadow_slice(const __grid_constant__ PtA
     f3 axis_u = mk(0.0f), axis_v = mk(0.0f);
     set3(axis_u, u_axis, A.u.subsurface[2]);
     set3(axis_v, v_axis, A.u.subsurface[2]);
-    f3 gathered = 0.4f * mk(back.x, back.y, back.z);
+    // The products' sum rounded one way whether the loop is unrolled or not.
+    f3 gathered = mk(__fmul_rn(0.4f, back.x), __fmul_rn(0.4f, back.y), __fmul_rn(0.4f, back.z));
+#pragma unroll
     for (int i = 0; i < 4; i++) {
         f3 offset = (i & 1) == 0 ? axis_u : axis_v;
         offset *= i < 2 ? 1.0f : -1.0f;
         float4 t = lv_linear<GIVEN>(V, (prev + offset + 0.5f) / w.dims);
-        gathered += 0.15f * mk(t.x, t.y, t.z);
+        gathered = mk(fmaf(0.15f, t.x, gathered.x), fmaf(0.15f, t.y, gathered.y), fmaf(0.15f, t.z, gathered.z));
     }
     f3 indirect = gathered * mk(f.x, f.y, f.z);
     vol[at] = make_ushort4(f2h(indirect.x), f2h(indirect.y), f2h(indirect.z), f2h(direct));
@@ -687,9 +696,11 @@ cudaError_t launch_shadow_sweep(const PtArgs& a, ushort4* vol, int sx, int sy, i
     for (int i = 0; i < n; i++) {
         int slice = sign > 0 ? n - 1 - i : i;
         if (factors) {
-            // Programmatic dependent launch. A sweep of 126 x 122 x 94 texels along x, y,
-            // z: 1.14, 0.78, 0.77 ms; with launch_dependents and loads from L2 1.82,
-            // 1.04, 1.14; plain launches that take the factors themselves 2.13, 1.99, 1.88.
+            // Programmatic dependent launch. A sweep of 126 x 122 x 94 texels towards the
+            // default light, along x, y, z, factors and copy included: 0.86, 0.81, 0.63,
+            // 0.54 ms (plain launches that take the factors themselves 2.31, 2.13, 1.99,
+            // 1.88). With launch_dependents and loads past L1 the branching form took
+            // 1.37, 1.82, 1.04, 1.14 instead of its 1.12, 1.14, 0.78, 0.76.
             cudaLaunchConfig_t config = {};
             config.gridDim = g;
             config.blockDim = dim3(64);

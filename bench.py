@@ -273,11 +273,11 @@ def peaks():
 # DRAM bytes per frame of the path-tracing pass on the default workload
 # (head/neck 512x512x400, 1024x1024, studio light, UNORM16 density), estimated
 # from ncu: every stage launch of a 16-frame pass of the 256x256x200 / 512x512
-# case moves 279 MB per frame, 1.50 times that case's algorithmic bytes; times
-# this workload's algorithmic bytes (558 MB). The small case's volumes nearly
+# case moves 279 MB per frame, 1.59 times that case's algorithmic bytes; times
+# this workload's algorithmic bytes (531 MB). The small case's volumes nearly
 # fit in L2, so the volume traffic of the flight and shadow kernels is
 # under-counted.
-PASS_TRAFFIC_BYTES_PER_FRAME = 8.36e8
+PASS_TRAFFIC_BYTES_PER_FRAME = 8.45e8
 
 
 def ncu_traffic(args):

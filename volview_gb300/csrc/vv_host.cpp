@@ -1448,7 +1448,8 @@ static cudaError_t wf_state(vv_renderer::Pass& P, size_t cap, const Vol& v, cuda
         // late waves the three launches cost the chain more than the order
         // gives. Against a line at 16384: 1024^2 frame 8.21 -> 8.06 ms, a
         // 256^2 frame 3.20 -> 3.07, 16-frame passes alone 29.4 -> 29.0 and
-        // overlapped 22.9 -> 23.0 (within the runs' spread); 131072 the same.
+        // overlapped 22.9 -> 23.0 (within the runs' spread). At 32768 a 256^2 frame
+        // takes 3.18, and 131072 measures as 65536: the lowest line that gains in full.
         const char* e = std::getenv("VV_WF_BIN_MIN");
         w.bin_min = e ? (uint32_t)std::max(0, std::atoi(e)) : 65537u;
     }

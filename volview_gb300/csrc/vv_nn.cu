@@ -975,8 +975,10 @@ extern "C" vv_status vv_nn_l1_loss(const void* pred, int c, const float* target,
                                    float* loss, void* dpred, void* stream) {
     if (!pred || !target || !loss || !dpred || c < 3 || pixels <= 0 || !(grad_scale > 0.0f)) return VV_ERR_ARG;
     if (c % 8 == 0 && aligned16(pred) && aligned16(dpred)) {
-        k_l1_loss_q<<<(unsigned)std::min<long>((pixels + 255) / 256, 304), 256, 0, (cudaStream_t)stream>>>((const uint4*)pred, c / 8, target, pixels,
-                                                                           grad_scale, loss, (uint4*)dpred);
+        // At most 304 blocks, two per SM: each adds once to the one word of the loss.
+        const unsigned grid = (unsigned)std::min<long>((pixels + 255) / 256, 304);
+        k_l1_loss_q<<<grid, 256, 0, (cudaStream_t)stream>>>((const uint4*)pred, c / 8, target, pixels, grad_scale, loss,
+                                                            (uint4*)dpred);
         return launched();
     }
     k_l1_loss<<<blocks(pixels, 256), 256, 0, (cudaStream_t)stream>>>((const __half*)pred, c, target, pixels,
